@@ -13,6 +13,7 @@
 #include "ecl_mst.h"
 #include "internal.h"
 #include "mst_device.cuh"
+#include "rounds_device.cuh"
 #include "batch_device.cuh"
 #include <functional>
 #include <vector>
@@ -104,7 +105,8 @@ struct ecl_mst_ctx {
   int first_v_cap = 0;
   DevState* st = nullptr;
   DevState* st_host = nullptr;  // pinned
-  int round_grid = 0;
+  int round_grid = 0;  // most co-resident CTAs of k_round
+  int abl_grid = 0;    // the same of k_rounds (ablation variants)
   // device CSR + output for host-buffer runs (allocated on first use)
   int* d_nindex = nullptr;
   int* d_nlist = nullptr;
@@ -325,10 +327,11 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   for (auto& e : c->ev)
     if ((st = cuda_status(cudaEventCreate(&e)))) return fail(st);
   // every CTA of a round pass writes one segment of the round's output list
-  c->round_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, c->sm_count), kMaxRoundCtas);
+  c->round_grid = std::min(coop_grid((const void*)k_round, kBorThreads, c->sm_count), kMaxRoundCtas);
+  c->abl_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, c->sm_count), kMaxRoundCtas);
   c->vertex_grid = coop_grid((const void*)k_rounds_vertex, kRoundThreads, c->sm_count);
   if ((st = prepare_scan_kernels())) return fail(st);
-  if (c->round_grid <= 0 || c->vertex_grid <= 0) return fail(ECL_ERR_CUDA);
+  if (c->round_grid <= 0 || c->abl_grid <= 0 || c->vertex_grid <= 0) return fail(ECL_ERR_CUDA);
   *out = c;
   return ECL_OK;
 }
@@ -435,11 +438,6 @@ extern "C" int ecl_mst_ctx_sync(ecl_mst_ctx* c) {
 
 namespace {
 
-int launch_coop(const void* fn, int grid, int threads, void* arg, cudaStream_t s) {
-  void* args[] = {arg};
-  return cuda_status(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, 0, s));
-}
-
 // Opt the scan variants into their dynamic shared memory (once per device).
 int prepare_scan_kernels() {
   ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kLight, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<4>()));
@@ -500,6 +498,40 @@ int launch_scans(ecl_mst_ctx* c, bool device_split, int split, const ScanArgs& s
     ECL_CUDA_TRY(cudaStreamWaitEvent(s, c->scan_join[i], 0));
   }
   return ECL_OK;
+}
+
+// One phase's Boruvka rounds: the grid-wide kernel, then the cluster kernel
+// that ends the phase. The ablation switches run the variants kept in
+// k_rounds. `per_sm`: the caller's limit on CTAs per SM (0 = none).
+int enqueue_rounds(const RoundArgs& ra, int edges, int sm_count, int per_sm, int round_grid, int abl_grid,
+                   cudaStream_t s, const cudaAccessPolicyWindow* win) {
+  const int limit = per_sm > 0 ? per_sm * sm_count : INT_MAX;
+  if (ra.abl) {
+    const int grid = std::max(1, std::min({abl_grid, limit, (edges / 2 + kRoundThreads - 1) / kRoundThreads + 1}));
+    return launch_ex(k_rounds, grid, kRoundThreads, 0, s, true, win, ra);
+  }
+  constexpr int tile = kBorThreads * kBorEpt;
+  BorArgs ba{};
+  ba.phase = ra.phase;
+  ba.nodes = ra.nodes;
+  ba.list = ra.wl0;
+  ba.wl0 = ra.wl0;
+  ba.wl1 = ra.wl1;
+  ba.wl_cap = ra.wl_cap;
+  ba.parent = ra.parent;
+  ba.minv = ra.minv0;
+  ba.roots0 = reinterpret_cast<int*>(ra.minv1);  // the second min array's space holds the root lists
+  ba.roots1 = ba.roots0 + ra.nodes;
+  ba.inMST = ra.inMST;
+  ba.st = ra.st;
+  ba.solo = ra.small_tail;
+  ba.tail = ra.small_tail ? std::max(ra.small_tail, kTailEntries) : 0u;
+  ba.min_tiles = ra.min_tiles;
+  ba.count_atomics = ra.count_atomics;
+  const int grid = std::max(1, std::min({round_grid, limit, (edges / 2 + tile - 1) / tile + 1}));
+  const int st = launch_ex(k_round, grid, kBorThreads, 0, s, true, win, ba);
+  if (st) return st;
+  return launch_ex(k_round_tail, kTailCtas, kTailThreads, 0, s, false, win, ba);
 }
 
 // The L2 access-policy window of a solve (ECL_FLAG_L2_PERSIST): the packed
@@ -633,9 +665,6 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   // each round, which one CTA of a small tail would do alone
   if (ra.abl & kAblKeepEnds) ra.small_tail = 0;
   ra.min_tiles = o->round_min_tiles < 0 ? 0 : (o->round_min_tiles == 0 ? kDefaultMinTiles : o->round_min_tiles);
-  int rmax = c->round_grid;
-  if (o->ctas_per_sm > 0) rmax = std::min(rmax, o->ctas_per_sm * c->sm_count);
-  const int rgrid = std::max(1, std::min(rmax, (m / 2 + kRoundThreads - 1) / kRoundThreads + 1));
   if (o->flags & ECL_FLAG_NO_EDGE_BASED) {
     // vertex-centric rounds straight over the CSR: no scans, no worklists
     if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[5], s));
@@ -659,9 +688,7 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   if ((st = launch_scans<kLight>(c, device_split, split, sa, s, nullptr))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   ra.phase = 0;
-  if (win_all) st = launch_ex(k_rounds, rgrid, kRoundThreads, 0, s, true, win_all, ra);
-  else st = launch_coop((const void*)k_rounds, rgrid, kRoundThreads, &ra, s);
-  if (st) return st;
+  if ((st = enqueue_rounds(ra, m, c->sm_count, o->ctas_per_sm, c->round_grid, c->abl_grid, s, win_all))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[2], s));
   const int fgrid = (int)std::min<int64_t>(((int64_t)n + kThreads - 1) / kThreads, (int64_t)c->sm_count * 16);
   if (win_par) {
@@ -676,9 +703,7 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   if ((st = launch_scans<kHeavy>(c, device_split, split, sa, s, win_par))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[3], s));
   ra.phase = 1;
-  if (win_all) st = launch_ex(k_rounds, rgrid, kRoundThreads, 0, s, true, win_all, ra);
-  else st = launch_coop((const void*)k_rounds, rgrid, kRoundThreads, &ra, s);
-  if (st) return st;
+  if ((st = enqueue_rounds(ra, m, c->sm_count, o->ctas_per_sm, c->round_grid, c->abl_grid, s, win_all))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[4], s));
   return ECL_OK;
 }
@@ -1122,7 +1147,7 @@ struct NaDevice {
   bool ready = false;
   unsigned char* base = nullptr;  // device address of g_na_scratch on this device
   int sm_count = 0;
-  int round_grid = 0;
+  int round_grid = 0, abl_grid = 0;
 };
 constexpr int kNaMaxDevices = 64;
 NaDevice g_na_dev[kNaMaxDevices];
@@ -1144,10 +1169,11 @@ int na_setup(int dev, NaDevice** out) {
     ECL_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return ECL_ERR_UNSUPPORTED;
     ECL_CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
-    d.round_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, d.sm_count), kMaxRoundCtas);
+    d.round_grid = std::min(coop_grid((const void*)k_round, kBorThreads, d.sm_count), kMaxRoundCtas);
+    d.abl_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, d.sm_count), kMaxRoundCtas);
     int ps = prepare_scan_kernels();
     if (ps) return ps;
-    if (d.round_grid <= 0) return ECL_ERR_CUDA;
+    if (d.round_grid <= 0 || d.abl_grid <= 0) return ECL_ERR_CUDA;
     d.ready = true;
   }
   *out = &d;
@@ -1240,16 +1266,16 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   if (o.flags & ECL_FLAG_NO_SMALL_TAIL) ra.small_tail = 0;
   ra.count_atomics = (o.flags & ECL_FLAG_STATS) ? 1 : 0;
   ra.abl = round_ablation(o.flags);
-  const int rgrid = std::max(1, std::min(d->round_grid, (m / 2 + kRoundThreads - 1) / kRoundThreads + 1));
+  ra.min_tiles = kDefaultMinTiles;
   if ((st = launch_scan<kLight>(scan_ept(split), sa, s))) return st;
   ra.phase = 0;
-  if ((st = launch_coop((const void*)k_rounds, rgrid, kRoundThreads, &ra, s))) return st;
+  if ((st = enqueue_rounds(ra, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
   const int fgrid = (int)std::min<int64_t>(((int64_t)n + kThreads - 1) / kThreads, (int64_t)d->sm_count * 16);
   k_flatten<<<std::max(fgrid, 1), kThreads, 0, s>>>(parent, n, dst);
   ECL_CUDA_TRY(cudaGetLastError());
   if ((st = launch_scan<kHeavy>(heavy_ept(split), sa, s))) return st;
   ra.phase = 1;
-  if ((st = launch_coop((const void*)k_rounds, rgrid, kRoundThreads, &ra, s))) return st;
+  if ((st = enqueue_rounds(ra, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
   // Report device-side errors (malformed CSR, worklist overflow) to the caller.
   unsigned err = 0;
   ECL_CUDA_TRY(cudaMemcpyAsync(&err, &dst->error, sizeof(err), cudaMemcpyDeviceToHost, s));

@@ -17,12 +17,14 @@
 //                 warps and CTAs (the reference's thread/warp degree split,
 //                 :167/:185, becomes the entries-per-lane E). Also zeroes
 //                 inMST. Appends are warp-aggregated, reserved in chunks.
-//   k_rounds      all Boruvka rounds of the phase in one cooperative launch
-//                 (kernel1, kernel2, kernel3 per round, bounded grid
-//                 barriers, no host round trip per round).
+//   k_round       the phase's Boruvka rounds in one cooperative launch
+//                 (rounds_device.cuh: kernel1, kernel2, kernel3 per round,
+//                 bounded grid barriers, no host round trip per round), and
+//   k_round_tail  its last rounds on one thread-block cluster. The ablation
+//                 switches run the variants in k_rounds instead.
 //   k_flatten     parent[v] = root(v) once after the light phase
 //   k_scan<H,E>   initWL<false>: keeps heavy entries across light trees
-//   k_rounds      heavy phase
+//   k_round, k_round_tail   heavy phase
 #pragma once
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>

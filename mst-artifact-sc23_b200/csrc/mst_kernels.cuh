@@ -88,6 +88,19 @@ struct FeatPart {
   }
 };
 
+// The state a phase's rounds are in at the top of a round (kept in the control
+// block where the cluster kernel takes over from the grid).
+struct BorState {
+  unsigned W;  // entries of the list read next
+  unsigned C;  // live roots (0 before the first roots pass)
+  int r;       // round
+  int k;       // compactions so far
+  int nseg;    // segments of the list (0 = dense)
+  int flips;   // roots passes so far
+  int first;   // no offer pass yet
+  int skip;    // the tree that offers nothing, -1 = none
+};
+
 // Control block of one solve, zeroed before every solve.
 struct DevState {
   int threshold;       // light phase keeps w <= threshold
@@ -114,6 +127,9 @@ struct DevState {
   // barrier that ends the pass, read after it).
   unsigned seg_cnt[kMaxRoundCtas];
   unsigned seg_off[kMaxRoundCtas];
+  unsigned root_cnt[2][3];  // [phase][pass % 3] = live roots a roots pass kept
+  BorState resume;          // where the cluster kernel goes on with the phase
+  int giant;                // the light phase's largest tree (by a vote of sampled vertices)
 };
 
 __device__ __forceinline__ u64 globaltimer_ns() {
