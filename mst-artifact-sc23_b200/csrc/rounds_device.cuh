@@ -468,6 +468,9 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
       b.W = 0;
       break;
     }
+    // The next round's segment table is read here, two barriers before any CTA
+    // can be at the end of that round's offer pass and publish new segments.
+    if (!fresh) bor_seg_load<T>(s, st, (int)stride);
     // ---- mark: the first round's scan list, or this CTA's own segment
     {
       const unsigned cnt = fresh ? W : s.cursor;
@@ -543,10 +546,8 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     b.flips++;
     if (b.skip >= 0) b.skip = ld_ca(a.parent + b.skip);
     if (!fresh) {
-      bor_seg_load<T>(s, st, (int)stride);
       b.nseg = (int)stride;
       b.k++;
-      __syncthreads();
     }
     b.first = 0;
     b.W = W2;
