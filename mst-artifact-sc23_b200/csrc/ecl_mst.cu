@@ -14,7 +14,8 @@
 #include "internal.h"
 #include "mst_device.cuh"
 #include "rounds_device.cuh"
-#include "batch_device.cuh"
+#include "group_device.cuh"
+#include "cluster_device.cuh"
 #include <functional>
 #include <vector>
 
@@ -35,6 +36,14 @@ constexpr unsigned kDefaultSmallTail = 4096;
 constexpr int kDefaultMinTiles = 1;  // round CTAs kept: one per tile of the round's worklist
 constexpr int64_t kWlSlack = 1 << 19;  // worklist slots beyond `edges` (scan chunk tails)
 constexpr int kLearnedMinEdges = 1 << 20;
+// Single graphs up to this many entries are solved in one launch (k_group):
+// RMAT-14 156 us against 200 with a launch per pass, ER 200k 295 against 327,
+// the 1000 x 1000 grid (4.0M entries) 456 against 481.
+constexpr int kGroupEdges = 1 << 22;
+// and of up to this many entries by one cluster (k_cluster), alone on one CTA
+// up to kClusterShare
+constexpr int kClusterEdges = 1 << 16;
+constexpr int kClusterShare = 1 << 14;
 }  // namespace
 
 // =================================================================== host
@@ -107,6 +116,7 @@ struct ecl_mst_ctx {
   DevState* st_host = nullptr;  // pinned
   int round_grid = 0;  // most co-resident CTAs of k_round
   int abl_grid = 0;    // the same of k_rounds (ablation variants)
+  int group_grid = 0;  // the same of k_group
   // device CSR + output for host-buffer runs (allocated on first use)
   int* d_nindex = nullptr;
   int* d_nlist = nullptr;
@@ -142,7 +152,7 @@ int cuda_status(cudaError_t e) {
 
 int device_error_status(unsigned err) {
   if (err & kErrTimeout) return ECL_ERR_TIMEOUT;
-  if (err & kErrFormat) return ECL_ERR_FORMAT;
+  if (err & (kErrFormat | kErrIds)) return ECL_ERR_FORMAT;
   if (err & kErrOverflow) return ECL_ERR_OVERFLOW;
   if (err & kErrRounds) return ECL_ERR_OVERFLOW;
   return ECL_OK;
@@ -199,7 +209,26 @@ int launch_ex(void (*kernel)(KArgs...), int grid, int threads, size_t smem, cuda
   return cuda_status(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
+// Launch `clusters` clusters of `size` CTAs.
+template <typename... KArgs, typename... Args>
+int launch_cluster(void (*kernel)(KArgs...), int size, int clusters, int threads, size_t smem, cudaStream_t s,
+                   Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size * clusters);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = size;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 int prepare_scan_kernels();
+int prepare_cluster_kernels();
 
 // Entries of the tile->vertex table buffer for up to `edges` CSR entries: the
 // table (tiles + 1) and the fill scan's chunk maxima.
@@ -329,9 +358,11 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   // every CTA of a round pass writes one segment of the round's output list
   c->round_grid = std::min(coop_grid((const void*)k_round, kBorThreads, c->sm_count), kMaxRoundCtas);
   c->abl_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, c->sm_count), kMaxRoundCtas);
+  c->group_grid = coop_grid((const void*)k_group, kGroupThreads, c->sm_count);
   c->vertex_grid = coop_grid((const void*)k_rounds_vertex, kRoundThreads, c->sm_count);
   if ((st = prepare_scan_kernels())) return fail(st);
-  if (c->round_grid <= 0 || c->abl_grid <= 0 || c->vertex_grid <= 0) return fail(ECL_ERR_CUDA);
+  if ((st = prepare_cluster_kernels())) return fail(st);
+  if (c->round_grid <= 0 || c->abl_grid <= 0 || c->group_grid <= 0 || c->vertex_grid <= 0) return fail(ECL_ERR_CUDA);
   *out = c;
   return ECL_OK;
 }
@@ -534,6 +565,61 @@ int enqueue_rounds(const RoundArgs& ra, int edges, int sm_count, int per_sm, int
   return launch_ex(k_round_tail, kTailCtas, kTailThreads, 0, s, false, win, ba);
 }
 
+// Opt the one-CTA kernels into their shared memory (once per device).
+int prepare_cluster_kernels() {
+  ECL_CUDA_TRY(cudaFuncSetAttribute(k_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmem));
+  ECL_CUDA_TRY(cudaFuncSetAttribute(k_batch_cluster<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmem));
+  return ECL_OK;
+}
+
+// CTAs of the cluster that solves a graph alone (k_cluster), 0 = k_group does.
+// One CTA up to kClusterShare entries and what its shared memory holds, else
+// one per half of that. Measured against k_group: ER of 1000 vertices 57 us
+// (one CTA) against 99, ER 4000 107 (4 CTAs) against 156, 16 000-vertex grid
+// (8 CTAs) 138 against 165; from 128K entries on k_group is the faster one.
+int cluster_ctas(int n, int m, unsigned wl_cap) {
+  if (m > kClusterEdges || n > kClusterEdges || (unsigned)m > wl_cap) return 0;
+  if (m <= kClusterShare && n <= kClVertices) return 1;
+  int c = 2;
+  while (c < kClMaxCtas && m > c * (kClusterShare / 2)) c *= 2;
+  return c;
+}
+
+int enqueue_cluster(ClArgs ca, int ctas, const mst_opts* o, cudaStream_t s) {
+  ca.mode = o->threshold_mode;
+  ca.explicit_thr = o->threshold;
+  ca.split = o->degree_split > 0 ? o->degree_split : kDefaultSplit;
+  ca.quantile = o->quantile;
+  ca.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
+  if (ctas == 1) return launch_cluster(k_cluster<true>, 1, 1, kClThreads, kClSmem, s, ca);
+  return launch_cluster(k_cluster<false>, ctas, 1, kClThreads, 0, s, ca);
+}
+
+// A whole solve in one launch (k_group), on one CTA per kGroupCtaTiles scan
+// tiles of the graph; `per_sm` is the caller's limit on CTAs per SM (0 = none)
+// and `wl_slack` what the worklists hold beyond the entries a scan can keep.
+// 1, 2, 4, 8 tiles per CTA: RMAT-14 163, 156, 162, 191 us; ER 200k 292, 295,
+// 309, 337; the 1000 x 1000 grid 455, 456, 454, 475.
+constexpr int kGroupCtaTiles = 2;
+int enqueue_group(GroupArgs ga, const mst_opts* o, unsigned wl_slack, int sm_count, int group_grid, cudaStream_t s,
+                  const cudaAccessPolicyWindow* win) {
+  constexpr int per_cta = kGroupCtaTiles * kGroupTile;
+  const int limit = o->ctas_per_sm > 0 ? o->ctas_per_sm * sm_count : INT_MAX;
+  const int grid = std::max(1, std::min({group_grid, limit, std::max((ga.edges + per_cta - 1) / per_cta,
+                                                                     (int)(((int64_t)ga.nodes + per_cta - 1) / per_cta))}));
+  ga.mode = o->threshold_mode;
+  ga.explicit_thr = o->threshold;
+  ga.split = o->degree_split > 0 ? o->degree_split : kDefaultSplit;
+  ga.quantile = o->quantile;
+  ga.solo = o->small_tail < 0 ? 0u : (o->small_tail == 0 ? kDefaultSmallTail : (unsigned)o->small_tail);
+  if (o->flags & ECL_FLAG_NO_SMALL_TAIL) ga.solo = 0;
+  ga.min_tiles = o->round_min_tiles < 0 ? 0 : (o->round_min_tiles == 0 ? kDefaultMinTiles : o->round_min_tiles);
+  ga.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
+  ga.chunk = std::min(256u, wl_slack / (unsigned)grid);
+  if (ga.chunk < 128) ga.chunk = 0;  // a warp may append 128 entries at once
+  return launch_ex(k_group, grid, kGroupThreads, 0, s, grid > 1, win, ga);
+}
+
 // The L2 access-policy window of a solve (ECL_FLAG_L2_PERSIST): the packed
 // min-slot and parent arrays (20n bytes; the min slots alone when the window
 // limit is smaller), with the share of lines the persisting set-aside can
@@ -589,6 +675,54 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   const bool l2 = (o->flags & ECL_FLAG_L2_PERSIST) != 0;
   const cudaAccessPolicyWindow* win_all = l2 && l2_window(c, sl, false, &w_all) ? &w_all : nullptr;
   const cudaAccessPolicyWindow* win_par = l2 && l2_window(c, sl, true, &w_par) ? &w_par : nullptr;
+  const bool one_launch = !lp && !round_ablation(o->flags) && !(o->flags & ECL_FLAG_NO_EDGE_BASED);
+  if (const int ctas = one_launch && o->ctas_per_sm == 0 && !(o->flags & ECL_FLAG_NO_SMALL_TAIL)
+                           ? cluster_ctas(n, m, c->wl_cap) : 0) {
+    ClArgs ca{};
+    ca.nodes = n;
+    ca.edges = m;
+    ca.nindex = g->nindex;
+    ca.nlist = g->nlist;
+    ca.eweight = g->eweight;
+    ca.inMST = d_inMST;
+    ca.wl0 = c->wl[0];
+    ca.wl1 = c->wl[1];
+    ca.parent = sl.parent;
+    ca.minv = sl.minv0;
+    ca.st = c->st;
+    if (timed)  // one launch: all of it counts as rounds
+      for (int k : {5, 1}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    const int r = enqueue_cluster(ca, ctas, o, s);
+    if (r) return r;
+    if (timed)
+      for (int k : {2, 6, 3, 4}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    return ECL_OK;
+  }
+  if (m <= kGroupEdges && one_launch) {
+    GroupArgs ga{};
+    ga.nodes = n;
+    ga.edges = m;
+    ga.nindex = g->nindex;
+    ga.nlist = g->nlist;
+    ga.eweight = g->eweight;
+    ga.inMST = d_inMST;
+    ga.parent = sl.parent;
+    ga.minv = sl.minv0;
+    ga.roots0 = reinterpret_cast<int*>(sl.minv1);
+    ga.roots1 = ga.roots0 + n;
+    ga.wl0 = c->wl[0];
+    ga.wl1 = c->wl[1];
+    ga.wl_cap = c->wl_cap;
+    ga.st = c->st;
+    if (timed)  // one launch: all of it counts as rounds
+      for (int k : {5, 1}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    const int r = enqueue_group(ga, o, c->wl_cap - (unsigned)(c->wl_full ? m : m / 2), c->sm_count, c->group_grid, s,
+                                win_all);
+    if (r) return r;
+    if (timed)
+      for (int k : {2, 6, 3, 4}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    return ECL_OK;
+  }
   PrepArgs pa{};
   pa.nodes = n;
   pa.edges = m;
@@ -1147,7 +1281,7 @@ struct NaDevice {
   bool ready = false;
   unsigned char* base = nullptr;  // device address of g_na_scratch on this device
   int sm_count = 0;
-  int round_grid = 0, abl_grid = 0;
+  int round_grid = 0, abl_grid = 0, group_grid = 0;
 };
 constexpr int kNaMaxDevices = 64;
 NaDevice g_na_dev[kNaMaxDevices];
@@ -1171,9 +1305,10 @@ int na_setup(int dev, NaDevice** out) {
     ECL_CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
     d.round_grid = std::min(coop_grid((const void*)k_round, kBorThreads, d.sm_count), kMaxRoundCtas);
     d.abl_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, d.sm_count), kMaxRoundCtas);
+    d.group_grid = coop_grid((const void*)k_group, kGroupThreads, d.sm_count);
     int ps = prepare_scan_kernels();
-    if (ps) return ps;
-    if (d.round_grid <= 0 || d.abl_grid <= 0) return ECL_ERR_CUDA;
+    if (ps || (ps = prepare_cluster_kernels())) return ps;
+    if (d.round_grid <= 0 || d.abl_grid <= 0 || d.group_grid <= 0) return ECL_ERR_CUDA;
     d.ready = true;
   }
   *out = &d;
@@ -1212,9 +1347,56 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   int4* wl0 = (int4*)(d->base + kNaOffWl0);
   int4* wl1 = (int4*)(d->base + kNaOffWl1);
   // The array keeps the previous call's contents: the control block (error
-  // word, worklist counters, barrier) must start at zero; k_prep initialises
-  // parent[] and both min arrays.
-  ECL_CUDA_TRY(cudaMemsetAsync(dst, 0, sizeof(DevState), s));
+  // word, worklist counters, barrier) must start at zero (k_cluster clears it
+  // itself); the kernels initialise parent[] and the min arrays.
+  const int ctas = round_ablation(o.flags) || (o.flags & ECL_FLAG_NO_SMALL_TAIL)
+                       ? 0 : cluster_ctas(n, m, (unsigned)kNaWlCap);
+  if (!ctas) ECL_CUDA_TRY(cudaMemsetAsync(dst, 0, sizeof(DevState), s));
+  auto finish = [&]() -> int {
+    // Report device-side errors (malformed CSR, worklist overflow) to the caller.
+    unsigned err = 0;
+    ECL_CUDA_TRY(cudaMemcpyAsync(&err, &dst->error, sizeof(err), cudaMemcpyDeviceToHost, s));
+    ECL_CUDA_TRY(cudaStreamSynchronize(s));
+    return device_error_status(err);
+  };
+  if (ctas) {
+    ClArgs ca{};
+    ca.nodes = n;
+    ca.edges = m;
+    ca.nindex = g->nindex;
+    ca.nlist = g->nlist;
+    ca.eweight = g->eweight;
+    ca.inMST = d_inMST;
+    ca.wl0 = wl0;
+    ca.wl1 = wl1;
+    ca.parent = parent;
+    ca.minv = minv0;
+    ca.st = dst;
+    if ((st = enqueue_cluster(ca, ctas, &o, s))) return st;
+    return finish();
+  }
+  if (!round_ablation(o.flags)) {
+    GroupArgs ga{};
+    ga.nodes = n;
+    ga.edges = m;
+    ga.nindex = g->nindex;
+    ga.nlist = g->nlist;
+    ga.eweight = g->eweight;
+    ga.inMST = d_inMST;
+    ga.parent = parent;
+    ga.minv = minv0;
+    ga.roots0 = reinterpret_cast<int*>(minv1);
+    ga.roots1 = ga.roots0 + n;
+    ga.wl0 = wl0;
+    ga.wl1 = wl1;
+    ga.wl_cap = (unsigned)kNaWlCap;
+    ga.st = dst;
+    // within the stated limit a scan keeps at most m / 2 entries
+    o.ctas_per_sm = 0;
+    const unsigned slack = (unsigned)std::max<int64_t>(0, kNaWlCap - m / 2);
+    if ((st = enqueue_group(ga, &o, slack, d->sm_count, d->group_grid, s, nullptr))) return st;
+    return finish();
+  }
   const int split = o.degree_split > 0 ? o.degree_split : kDefaultSplit;
   const int tiles = (int)(((int64_t)m + kGran - 1) / kGran);
   PrepArgs pa{};
@@ -1276,11 +1458,7 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   if ((st = launch_scan<kHeavy>(heavy_ept(split), sa, s))) return st;
   ra.phase = 1;
   if ((st = enqueue_rounds(ra, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
-  // Report device-side errors (malformed CSR, worklist overflow) to the caller.
-  unsigned err = 0;
-  ECL_CUDA_TRY(cudaMemcpyAsync(&err, &dst->error, sizeof(err), cudaMemcpyDeviceToHost, s));
-  ECL_CUDA_TRY(cudaStreamSynchronize(s));
-  return device_error_status(err);
+  return finish();
 }
 
 // ============================================================== batched mode
@@ -1297,6 +1475,9 @@ constexpr int kDefaultLargeStreams = 4;  // measured: 957 large graphs of the mi
 
 }  // namespace
 
+// Size classes of a batch's small graphs (batch_small).
+constexpr int kBatchClasses = 4;
+
 struct ecl_batch_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -1304,14 +1485,17 @@ struct ecl_batch_ctx {
   int max_graphs = 0;
   int64_t max_nodes = 0, max_edges = 0;
   int cap = 0;        // per-CTA scratch: vertices and CSR entries
-  int small_grid = 0; // CTAs of the persistent kernel
+  // scratch for small_grid graphs of `cap` vertices and entries; a run divides
+  // it among the clusters of its size classes (at most sm_count / size each)
+  int small_grid = 0;
   int* parent_pool = nullptr;
   u64* minv_pool = nullptr;
   int4* wl_pool = nullptr;
-  long long* d_node_off = nullptr;
-  long long* d_edge_off = nullptr;
-  int* d_small = nullptr;
-  unsigned* d_queue = nullptr;
+  DevState* states = nullptr;   // a control block per cluster
+  GraphDesc* d_graphs = nullptr;
+  unsigned* d_queue = nullptr;  // one per size class
+  cudaStream_t cls_stream[kBatchClasses - 1] = {};  // the classes beside the first
+  cudaEvent_t cls_fork = nullptr, cls_join[kBatchClasses - 1] = {};
   DevState* st = nullptr;
   // grid-wide engines for the graphs beyond the cutoff, one per concurrent
   // stream: [0] is made with the context, the others when a solve asks for
@@ -1346,9 +1530,13 @@ extern "C" void ecl_batch_ctx_destroy(ecl_batch_ctx* c) {
   cudaFree(c->parent_pool);
   cudaFree(c->minv_pool);
   cudaFree(c->wl_pool);
-  cudaFree(c->d_node_off);
-  cudaFree(c->d_edge_off);
-  cudaFree(c->d_small);
+  for (cudaStream_t q : c->cls_stream)
+    if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t e : c->cls_join)
+    if (e) cudaEventDestroy(e);
+  if (c->cls_fork) cudaEventDestroy(c->cls_fork);
+  cudaFree(c->states);
+  cudaFree(c->d_graphs);
   cudaFree(c->d_queue);
   cudaFree(c->st);
   for (auto& e : c->ev)
@@ -1385,19 +1573,20 @@ extern "C" int ecl_batch_ctx_create(int device, int32_t max_graphs, int64_t max_
   if ((st = cuda_status(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device))))
     return fail(st);
   if ((st = cuda_status(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)))) return fail(st);
-  int per_sm = 0;
-  if ((st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_batch_small,
-                                                                      kThreads, 0))))
-    return fail(st);
-  c->small_grid = std::max(1, per_sm) * c->sm_count;
+  c->small_grid = 2 * c->sm_count;
+  if ((st = prepare_cluster_kernels())) return fail(st);
   const size_t ctas = (size_t)c->small_grid, cap = (size_t)c->cap;
   if ((st = cuda_status(cudaMalloc(&c->parent_pool, ctas * cap * sizeof(int))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->minv_pool, ctas * 2 * cap * sizeof(u64))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->minv_pool, ctas * cap * sizeof(u64))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->wl_pool, ctas * 2 * cap * sizeof(int4))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->d_node_off, 2 * (size_t)max_graphs * sizeof(long long))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->d_edge_off, 2 * (size_t)max_graphs * sizeof(long long))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->d_small, (size_t)max_graphs * sizeof(int))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->d_queue, sizeof(unsigned))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->states, ctas * sizeof(DevState))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->d_graphs, (size_t)max_graphs * sizeof(GraphDesc))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->d_queue, kBatchClasses * sizeof(unsigned))))) return fail(st);
+  for (auto& q : c->cls_stream)
+    if ((st = cuda_status(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking)))) return fail(st);
+  if ((st = cuda_status(cudaEventCreateWithFlags(&c->cls_fork, cudaEventDisableTiming)))) return fail(st);
+  for (auto& e : c->cls_join)
+    if ((st = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->st, sizeof(DevState))))) return fail(st);
   for (auto& e : c->ev)
     if ((st = cuda_status(cudaEventCreate(&e)))) return fail(st);
@@ -1412,10 +1601,90 @@ extern "C" int ecl_batch_ctx_create(int device, int32_t max_graphs, int64_t max_
 
 namespace {
 
-// Per-graph descriptors for the persistent kernel use the "nodes / edges"
-// form: node_off[g] = nindex_off[g] - g keeps nindex at node_off[g] + g, and
-// edge_off[g + 1] - edge_off[g] must give edges[g], so the kernel gets its own
-// compact offset arrays built here (one entry per small graph, in queue order).
+// The graphs solved by clusters. A graph's cluster has two CTAs or more if one
+// cannot hold its vertices (kClVertices), and as many as its share of the
+// batch's entries asks for, so that no graph is worked on much longer than an
+// even split of the batch over the chip takes (twice that share, rounded up to
+// 1, 2, 4 or 8): a batch of thousands runs one CTA to a graph, a few graphs run
+// on as much of the chip as they can use. Largest first within a class; the
+// classes run side by side, the largest clusters launched first. 398 graphs of
+// 1000 to 60 000 vertices: 1.9 ms against 7.1 with one CTA to every graph.
+int batch_small(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& small, uint8_t* d_inMST,
+                const mst_opts* o, cudaStream_t s) {
+  const int S = (int)small.size();
+  int64_t total = 0;
+  for (int g : small) total += b->edges[g];
+  const int64_t share = std::max<int64_t>(kClTile, total / (2 * c->sm_count));
+  auto class_of = [&](int g) {  // class k: 8 >> k CTAs
+    int k = b->nodes[g] > kClVertices ? kBatchClasses - 2 : kBatchClasses - 1;
+    while (k > 0 && b->edges[g] > (8 >> k) * share) k--;
+    return k;
+  };
+  std::vector<int> order(small);
+  std::vector<int> cls(b->num_graphs);
+  for (int g : small) cls[g] = class_of(g);
+  std::sort(order.begin(), order.end(), [&](int x, int y) {
+    return cls[x] != cls[y] ? cls[x] < cls[y] : b->edges[x] > b->edges[y];
+  });
+  std::vector<GraphDesc> descs(S);
+  int first[kBatchClasses + 1] = {};
+  for (int i = 0; i < S; i++) {
+    const int g = order[i];
+    descs[i] = GraphDesc{b->nindex_off[g], b->edge_off[g], b->nodes[g], b->edges[g]};
+    for (int k = cls[g] + 1; k <= kBatchClasses; k++) first[k] = i + 1;
+  }
+  ECL_CUDA_TRY(cudaMemsetAsync(c->d_queue, 0, kBatchClasses * sizeof(unsigned), s));
+  ECL_CUDA_TRY(cudaMemcpyAsync(c->d_graphs, descs.data(), (size_t)S * sizeof(GraphDesc), cudaMemcpyHostToDevice, s));
+  BatchArgs ba{};
+  ba.nindex = b->nindex;
+  ba.nlist = b->nlist;
+  ba.eweight = b->eweight;
+  ba.inMST = d_inMST;
+  ba.st = c->st;
+  ba.mode = o->threshold_mode == ECL_THRESH_LEARNED ? ECL_THRESH_HEURISTIC : o->threshold_mode;
+  ba.explicit_thr = o->threshold;
+  ba.quantile = o->quantile;
+  ba.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
+  const int64_t pool = (int64_t)c->small_grid * c->cap;
+  int64_t used = 0;  // pool entries given out
+  int states = 0, forked = 0;
+  ECL_CUDA_TRY(cudaEventRecord(c->cls_fork, s));
+  for (int k = 0; k < kBatchClasses; k++) {
+    const int count = first[k + 1] - first[k], size = 8 >> k;
+    if (count <= 0) continue;
+    int64_t cap = 1;
+    for (int i = first[k]; i < first[k + 1]; i++)
+      cap = std::max<int64_t>(cap, std::max(descs[i].nodes, descs[i].edges));
+    cap = (cap + 3) & ~(int64_t)3;
+    // the classes after this one keep at least one cluster's worth of the pool
+    const int later = kBatchClasses - 1 - k;
+    const int64_t fit = (pool - later * ((int64_t)c->cap + 3) - used) / cap;
+    const int clusters = (int)std::min<int64_t>({(int64_t)count, (int64_t)std::max(1, c->sm_count / size), fit,
+                                                 (int64_t)c->small_grid - later - states});
+    ba.graphs = c->d_graphs + first[k];
+    ba.count = count;
+    ba.queue = c->d_queue + k;
+    ba.states = c->states + states;
+    ba.parent_pool = c->parent_pool + used;
+    ba.minv_pool = c->minv_pool + used;
+    ba.wl_pool = c->wl_pool + 2 * used;
+    ba.cap = cap;
+    used += clusters * cap;
+    states += clusters;
+    cudaStream_t q = s;
+    if (first[k + 1] < S) {  // the last class runs on the caller's stream
+      q = c->cls_stream[forked];
+      ECL_CUDA_TRY(cudaStreamWaitEvent(q, c->cls_fork, 0));
+    }
+    const int st = size == 1 ? launch_cluster(k_batch_cluster<true>, 1, clusters, kClThreads, kClSmem, q, ba)
+                             : launch_cluster(k_batch_cluster<false>, size, clusters, kClThreads, 0, q, ba);
+    if (st) return st;
+    if (q != s) ECL_CUDA_TRY(cudaEventRecord(c->cls_join[forked++], q));
+  }
+  for (int i = 0; i < forked; i++) ECL_CUDA_TRY(cudaStreamWaitEvent(s, c->cls_join[i], 0));
+  return ECL_OK;
+}
+
 int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const mst_opts* o,
                   cudaStream_t s, bool timed, ecl_batch_stats* stats) {
   const int G = b->num_graphs;
@@ -1431,53 +1700,12 @@ int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const 
     else large.push_back(g);
   }
   if (!large.empty() && !c->big[0]) return ECL_ERR_TOO_LARGE;
-  // largest first: the persistent kernel's tail then consists of small graphs
-  std::sort(small.begin(), small.end(), [&](int x, int y) { return b->edges[x] > b->edges[y]; });
-  // compact descriptors: small graph i -> (node_off, edge_off) pairs at i, i + 1
   const int S = (int)small.size();
-  std::vector<long long> noff(2 * (size_t)S), eoff(2 * (size_t)S);
-  std::vector<int> ids(S);
-  for (int i = 0; i < S; i++) {
-    const int g = small[i];
-    noff[2 * i] = b->nindex_off[g] - 2 * (long long)i;     // + id (= 2i) gives nindex_off
-    noff[2 * i + 1] = noff[2 * i] + b->nodes[g];
-    eoff[2 * i] = b->edge_off[g];
-    eoff[2 * i + 1] = b->edge_off[g] + b->edges[g];
-    ids[i] = 2 * i;
-  }
   ECL_CUDA_TRY(cudaMemsetAsync(c->st, 0, sizeof(DevState), s));
-  ECL_CUDA_TRY(cudaMemsetAsync(c->d_queue, 0, sizeof(unsigned), s));
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[0], s));
   if (S > 0) {
-    ECL_CUDA_TRY(cudaMemcpyAsync(c->d_node_off, noff.data(), noff.size() * sizeof(long long),
-                                 cudaMemcpyHostToDevice, s));
-    ECL_CUDA_TRY(cudaMemcpyAsync(c->d_edge_off, eoff.data(), eoff.size() * sizeof(long long),
-                                 cudaMemcpyHostToDevice, s));
-    ECL_CUDA_TRY(cudaMemcpyAsync(c->d_small, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    BatchArgs ba;
-    ba.num_small = S;
-    ba.small_list = c->d_small;
-    ba.node_off = c->d_node_off;
-    ba.edge_off = c->d_edge_off;
-    ba.nindex = b->nindex;
-    ba.nlist = b->nlist;
-    ba.eweight = b->eweight;
-    ba.inMST = d_inMST;
-    ba.parent_pool = c->parent_pool;
-    ba.minv_pool = c->minv_pool;
-    ba.wl_pool = c->wl_pool;
-    ba.cap_n = c->cap;
-    ba.cap_m = c->cap;
-    ba.queue = c->d_queue;
-    ba.st = c->st;
-    ba.mode = o->threshold_mode == ECL_THRESH_LEARNED ? ECL_THRESH_HEURISTIC : o->threshold_mode;
-    ba.explicit_thr = o->threshold;
-    ba.quantile = o->quantile;
-    ba.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
-    ba.abl = round_ablation(o->flags);
-    const int grid = std::min(c->small_grid, S);
-    k_batch_small<<<grid, kThreads, 0, s>>>(ba);
-    ECL_CUDA_TRY(cudaGetLastError());
+    const int r = batch_small(c, b, small, d_inMST, o, s);
+    if (r) return r;
   }
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   bool replayed = false;

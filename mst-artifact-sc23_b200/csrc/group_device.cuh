@@ -1,0 +1,269 @@
+// A whole solve (initPM, initWL<true>, rounds, initWL<false>, rounds:
+// ECL-MST/ECL_MST.cu:305-340) in one launch, for a graph of up to kGroupEdges
+// entries, on a grid of as many CTAs as its size asks for. At these sizes the
+// ten launches of the separate kernels cost more than their work: an empty one
+// takes 5-8 us.
+#pragma once
+#include "rounds_device.cuh"
+
+namespace ecl {
+
+// 512 threads, two worklist entries each, two CTAs per SM: the scans and the
+// rounds together take 64 registers.
+constexpr int kGroupThreads = 512, kGroupEpt = 2, kGroupBlocks = 2;
+constexpr int kGroupTile = kGroupThreads * 4;  // CSR entries a CTA scans at a time
+
+struct GroupArgs {
+  int nodes, edges;
+  const int* nindex;
+  const int* nlist;
+  const int* eweight;
+  unsigned char* inMST;
+  int* parent;
+  u64* minv;
+  int* roots0;  // nodes entries each
+  int* roots1;
+  int4* wl0;
+  int4* wl1;
+  unsigned wl_cap;
+  unsigned chunk;  // worklist slots a CTA reserves at once, 0 = exactly what it needs
+  DevState* st;
+  int mode, explicit_thr, split;
+  float quantile;
+  unsigned solo;
+  int min_tiles;
+  int count_atomics;
+};
+
+struct GroupSmem {
+  union {
+    BorSmem bor;
+    int samp[4096];
+  };
+  u64 chunk;  // the CTA's current slots: first << 32 | given out
+  unsigned kept;
+};
+
+// The row that holds entry `jl` and the one that holds `jh` >= jl, found by
+// the whole warp: every step probes 32 rows of each range.
+__device__ __forceinline__ void warp_rows(const int* nindex, int n, int jl, int jh, int& lo, int& hi) {
+  const int lane = threadIdx.x & 31;
+  int len_l = n, len_h = n;
+  lo = hi = 0;
+  while (len_l > 1 || len_h > 1) {
+    const int sl = (len_l + 31) >> 5, sh = (len_h + 31) >> 5;
+    const int pl = lane * sl, ph = lane * sh;
+    const bool bl = pl < len_l && (lane == 0 || __ldg(nindex + lo + pl) <= jl);
+    const bool bh = ph < len_h && (lane == 0 || __ldg(nindex + hi + ph) <= jh);
+    const int kl = __popc(__ballot_sync(0xffffffffu, bl)) - 1, kh = __popc(__ballot_sync(0xffffffffu, bh)) - 1;
+    lo += kl * sl;
+    len_l = min(sl, len_l - kl * sl);
+    hi += kh * sh;
+    len_h = min(sh, len_h - kh * sh);
+  }
+}
+
+// initWL by a group: every thread takes four consecutive entries, looks for
+// the row of the first between the rows its warp spans, and walks on from
+// there; appends as tuples, in chunks of slots the CTA's warps share.
+template <int KIND>
+__device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, GroupSmem& sm) {
+  const int n = g.nodes, m = g.edges, lane = threadIdx.x & 31;
+  const int thr = g.st->threshold;
+  const bool vec = ((((uintptr_t)g.nlist) | ((uintptr_t)g.eweight)) & 15) == 0;
+  const bool zero_vec = (((uintptr_t)g.inMST) & 3) == 0;
+  unsigned* ctr = &g.st->wl_count[KIND][0];
+  if (threadIdx.x == 0) {
+    sm.chunk = g.chunk;
+    sm.kept = 0;
+  }
+  __syncthreads();
+  bool bad = false;
+  for (long long base = (long long)rank * kGroupTile; base < m; base += (long long)ctas * kGroupTile) {
+    const int jw = (int)base + ((int)threadIdx.x & ~31) * 4;  // the warp's first entry
+    if (jw >= m) continue;                                    // (whole warps)
+    const int j0 = jw + lane * 4, own = min(4, m - j0);       // own <= 0: none
+    int nb[4] = {}, w[4] = {};
+    if (own == 4 && vec) {
+      const int4 x = __ldg(reinterpret_cast<const int4*>(g.nlist + j0));
+      const int4 y = __ldg(reinterpret_cast<const int4*>(g.eweight + j0));
+      nb[0] = x.x; nb[1] = x.y; nb[2] = x.z; nb[3] = x.w;
+      w[0] = y.x; w[1] = y.y; w[2] = y.z; w[3] = y.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i < own) {
+          nb[i] = __ldg(g.nlist + j0 + i);
+          w[i] = __ldg(g.eweight + j0 + i);
+        }
+    }
+    if (KIND == kLight && own > 0) {
+      if (own == 4 && zero_vec) *reinterpret_cast<unsigned*>(g.inMST + j0) = 0u;
+      else
+        for (int i = 0; i < own; i++) g.inMST[j0 + i] = 0;
+    }
+    int lo, hi;
+    warp_rows(g.nindex, n, jw, min(jw + 127, m - 1), lo, hi);
+    while (lo < hi && own > 0) {  // the last row starting at or before j0
+      const int mid = lo + ((hi - lo + 1) >> 1);
+      if (__ldg(g.nindex + mid) <= j0) lo = mid;
+      else hi = mid - 1;
+    }
+    int v = lo, end = own > 0 ? __ldg(g.nindex + v + 1) : 0;
+    int4 e[4];
+    unsigned pass = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (i < own) {
+        while (j0 + i >= end && v < n - 1) end = __ldg(g.nindex + ++v + 1);
+        bad |= (unsigned)nb[i] >= (unsigned)n;
+        // one direction with a valid id (v < nb < n) as one unsigned compare
+        if ((unsigned)nb[i] - (unsigned)v - 1u < (unsigned)(n - v - 1) && (KIND == kLight ? w[i] <= thr : w[i] > thr))
+          pass |= 1u << i;
+      }
+      e[i] = make_int4(v, nb[i], w[i], j0 + i);
+    }
+    if (KIND == kHeavy) {  // the trees of both ends, all loads in flight together
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if ((pass >> i) & 1u) {
+          e[i].x = ld_ca(g.parent + e[i].x);
+          e[i].y = ld_ca(g.parent + e[i].y);
+        }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (e[i].x == e[i].y) pass &= ~(1u << i);
+    }
+    // the warp's slots
+    unsigned mask[4], total = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      mask[i] = __ballot_sync(0xffffffffu, (pass >> i) & 1u);
+      total += __popc(mask[i]);
+    }
+    if (!total) continue;
+    unsigned pos = 0, avail = 0, fresh = 0;
+    if (lane == 0) {
+      chunk_take(&sm.chunk, g.chunk, ctr, total, pos, avail, fresh, g.st, g.wl_cap);
+      atomicAdd(&sm.kept, total);
+    }
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    avail = __shfl_sync(0xffffffffu, avail, 0);
+    fresh = __shfl_sync(0xffffffffu, fresh, 0);
+    unsigned before = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const unsigned r = before + __popc(mask[i] & ((1u << lane) - 1u));
+      before += __popc(mask[i]);
+      if (!((pass >> i) & 1u)) continue;
+      const unsigned slot = r < avail ? pos + r : fresh + (r - avail);
+      if (slot >= g.wl_cap) atomicOr(&g.st->error, kErrOverflow);
+      else __stcg(g.wl0 + slot, e[i]);
+    }
+  }
+  if (bad) atomicOr(&g.st->error, kErrIds);  // a neighbour id outside [0, n)
+  __syncthreads();
+  const unsigned first = (unsigned)(sm.chunk >> 32);  // null entries in the slots not given out
+  for (unsigned p = (unsigned)sm.chunk + threadIdx.x; p < g.chunk; p += kGroupThreads)
+    if (first + p < g.wl_cap) g.wl0[first + p] = make_int4(-1, -1, 0, 0);
+  if (threadIdx.x == 0 && sm.kept) atomicAdd(&g.st->scan_kept[KIND], sm.kept);
+}
+
+// The rounds of one phase by the group, then the whole group again.
+template <class Sync>
+__device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, GroupSmem& sm) {
+  BorArgs a{};
+  a.phase = phase;
+  a.nodes = g.nodes;
+  a.list = a.wl0 = g.wl0;
+  a.wl1 = g.wl1;
+  a.wl_cap = g.wl_cap;
+  a.parent = g.parent;
+  a.minv = g.minv;
+  a.roots0 = g.roots0;
+  a.roots1 = g.roots1;
+  a.inMST = g.inMST;
+  a.st = g.st;
+  a.solo = g.solo;
+  a.min_tiles = g.min_tiles;
+  a.count_atomics = g.count_atomics;
+  BorState b = {};
+  b.W = min(ld_volatile(&g.st->wl_count[phase][0]), g.wl_cap);
+  b.first = 1;
+  b.skip = skip;
+  __syncthreads();  // the scan's use of the shared memory is over
+  bor_smem_init(sm.bor);
+  __syncthreads();
+  if (sy.rank == 0 && threadIdx.x == 0) g.st->t_round_start[phase] = globaltimer_ns();
+  bool left;
+  bor_rounds<kGroupThreads, kGroupEpt, true>(a, b, true, sy, sm.bor, left);
+  if (sy.rank == 0 && threadIdx.x == 0) g.st->rounds[phase] = b.r;
+  return sy.regroup(left, (unsigned)phase + 1u);
+}
+
+// One solve; the control block's counters are zero. False if a barrier timed
+// out. Every thread of the group calls this.
+template <class Sync>
+__device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
+  DevState* st = g.st;
+  const unsigned rank = sy.rank, ctas = sy.active, tid = threadIdx.x;
+  const unsigned gid = rank * kGroupThreads + tid, stride = ctas * kGroupThreads;
+  const int n = g.nodes, m = g.edges;
+  if (m == 0) return true;
+  if (rank == 0) {
+    PrepArgs pa{};
+    pa.nodes = n;
+    pa.edges = m;
+    pa.eweight = g.eweight;
+    pa.mode = g.mode;
+    pa.explicit_thr = g.explicit_thr;
+    pa.split = g.split;
+    pa.quantile = g.quantile;
+    pa.st = st;
+    choose_threshold(pa, sm.samp);
+  }
+  bool bad = false;
+  for (unsigned v = gid; v < (unsigned)n; v += stride) {
+    g.parent[v] = (int)v;
+    g.minv[v] = kNoEdge;
+    const int b = __ldg(g.nindex + v), e = __ldg(g.nindex + v + 1);
+    bad |= b < 0 || e < b || e > m;
+  }
+  if (gid == 0) bad |= __ldg(g.nindex) != 0 || __ldg(g.nindex + n) != m;
+  if (bad) atomicOr(&st->error, kErrFormat);
+  if (!sy.sync()) return false;
+  if (ld_volatile(&st->error) & kErrFormat) return true;  // only set before the barrier: the whole group
+  group_scan<kLight>(g, rank, ctas, sm);
+  if (!sy.sync()) return false;
+  const int filtered = st->filtered;
+  if (!group_rounds(g, 0, -1, sy, sm)) return false;
+  if (!filtered) return true;
+  // parent[v] = root(v), and the tree most entries point into (a vote of 32)
+  for (unsigned v = gid; v < (unsigned)n; v += stride) {
+    const int p = __ldcg(g.parent + v);
+    int r = p;
+    for (int x = ld_ca(g.parent + r); x != r; x = ld_ca(g.parent + r)) r = x;
+    if (r != p) __stcg(g.parent + v, r);
+  }
+  if (gid < 32) {
+    int v = __ldg(g.nlist + (unsigned)(((u64)uf_prio((int)gid + 1) * (u64)m) >> 32));
+    v = (unsigned)v < (unsigned)n ? v : 0;
+    const int r = find_ro(v, g.parent);
+    const unsigned same = __popc(__match_any_sync(0xffffffffu, r));
+    if (same == __reduce_max_sync(0xffffffffu, same)) st->giant = r;  // any of the largest groups
+  }
+  if (!sy.sync()) return false;
+  const int giant = (int)ld_volatile((const unsigned*)&st->giant);
+  group_scan<kHeavy>(g, rank, ctas, sm);
+  if (!sy.sync()) return false;
+  return group_rounds(g, 1, giant, sy, sm);
+}
+
+__global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) k_group(GroupArgs g) {
+  __shared__ GroupSmem sm;
+  GridSync sy;
+  sy.init(g.st, &g.st->bar[0]);
+  group_solve(g, sy, sm);
+}
+
+}  // namespace ecl

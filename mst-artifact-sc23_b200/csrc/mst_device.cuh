@@ -37,7 +37,7 @@
 
 namespace ecl {
 
-constexpr int kThreads = 512;          // threads of the prep, flatten and batch kernels
+constexpr int kThreads = 512;          // threads of the prep and flatten kernels
 constexpr int kGran = 128;             // entries per tile->vertex table step (the smallest scan warp range)
 // Round CTAs of 1024 threads, two per SM (measured on RMAT-22: 2.4 % faster
 // with the learned schedule and 4.6 % with the heuristic one than 512 x 4;
@@ -204,31 +204,27 @@ __device__ void choose_threshold(const PrepArgs& a, int* samp) {
     return;
   }
   if (mode == ECL_THRESH_HEURISTIC) {
-    if (tid == 0) {
-      if (edges / nodes < 4) {
-        st->filtered = 0;
-        st->threshold = INT_MAX;
-      } else {
-        int s[20];
-        const int ns = edges < 20 ? edges : 20;
-        for (int i = 0; i < ns; i++) {
-          unsigned val = (unsigned)i;
-          val = ((val >> 16) ^ val) * 0x45d9f3bu;
-          val = ((val >> 16) ^ val) * 0x45d9f3bu;
-          val = (val >> 16) ^ val;
-          s[i] = a.eweight[val % (unsigned)edges];
+    if (tid < 32) {  // one warp: a lane per sample, its rank by counting
+      const int ns = edges < 20 ? edges : 20;
+      unsigned val = (unsigned)tid;
+      val = ((val >> 16) ^ val) * 0x45d9f3bu;
+      val = ((val >> 16) ^ val) * 0x45d9f3bu;
+      val = (val >> 16) ^ val;
+      const bool filter = edges / nodes >= 4;
+      const int x = filter && tid < ns ? a.eweight[val % (unsigned)edges] : INT_MAX;
+      int rank = 0;
+      for (int i = 0; i < ns; i++) {
+        const int y = __shfl_sync(0xffffffffu, x, i);
+        rank += y < x || (y == x && i < tid);
+      }
+      if (!filter) {
+        if (tid == 0) {
+          st->filtered = 0;
+          st->threshold = INT_MAX;
         }
-        for (int i = 1; i < ns; i++) {
-          const int x = s[i];
-          int k = i - 1;
-          while (k >= 0 && s[k] > x) {
-            s[k + 1] = s[k];
-            k--;
-          }
-          s[k + 1] = x;
-        }
+      } else if (tid < ns && rank == min(19, (int)(3.0 * nodes * ns / edges))) {
         st->filtered = 1;
-        st->threshold = s[min(19, (int)(3.0 * nodes * ns / edges))];
+        st->threshold = x;
       }
     }
     return;
@@ -789,7 +785,7 @@ __global__ void __launch_bounds__(kThreads) k_flatten(int* parent, int n, const 
 // every entry's parent read, min-slot guard read, atomicMin and reset on one
 // L2 address; these small direct-mapped tables absorb the repeats per CTA.
 struct RoundSmem {
-  ReserveSmem rs;            // the batch kernel's CTA scans
+  ReserveSmem rs;            // the CTA's warp totals
   unsigned cursor;           // entries this CTA kept so far in the current find/min pass
   int seg_n;                 // segments of the list the passes read (1 = dense from seg_off[0])
   unsigned seg_q[kMaxRoundCtas + 1];  // entries in the segments before b (seg_q[seg_n] = all)

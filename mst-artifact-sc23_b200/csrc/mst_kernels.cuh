@@ -17,7 +17,9 @@ enum : unsigned {
   kErrFormat = 1u,    // nindex not monotone / out of range, or nlist id >= nodes
   kErrOverflow = 2u,  // a worklist or descriptor buffer ran out of room
   kErrTimeout = 4u,   // a grid barrier waited past its limit
-  kErrRounds = 8u     // more Boruvka rounds than ECL_MAX_ROUNDS
+  kErrRounds = 8u,    // more Boruvka rounds than ECL_MAX_ROUNDS
+  kErrIds = 16u       // nlist id out of range, found by a group's scan (k_group): a bit of
+                      // its own, as the group leaves together on kErrFormat
 };
 
 // Most CTAs a round-kernel launch may have: each CTA of a find/min pass
@@ -129,6 +131,10 @@ struct DevState {
   unsigned seg_off[kMaxRoundCtas];
   unsigned root_cnt[2][3];  // [phase][pass % 3] = live roots a roots pass kept
   BorState resume;          // where the cluster kernel goes on with the phase
+  unsigned bar[2];          // GridSync counters: k_round's by phase; k_group's
+  unsigned gate;            // the last gate opened (GridSync::regroup)
+  unsigned gate_target;
+  unsigned graph;           // batch: the graph the cluster works on
   int giant;                // the light phase's largest tree (by a vote of sampled vertices)
 };
 
@@ -269,6 +275,14 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, unsign
 __device__ __forceinline__ int ld_cg_hint(const int* p, u64 policy) {
   int v;
   asm volatile("ld.global.cg.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
+  return v;
+}
+
+// 32-bit global load through L1, for data that no CTA writes between two
+// barriers (or where an older value will do).
+__device__ __forceinline__ int ld_ca(const int* p) {
+  int v;
+  asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 

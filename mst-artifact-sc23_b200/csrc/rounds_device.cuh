@@ -54,6 +54,44 @@ struct BorArgs {
   int count_atomics;
 };
 
+// Slots for `total` entries of a list that a CTA's warps append to, out of the
+// chunk they share (`word`: first slot << 32 | slots given out; more given out
+// than the `chunk` slots it holds: a warp is fetching the next one). The first
+// `avail` of them start at `pos`, the others at `fresh`. One thread of a warp
+// calls this; total <= chunk. A chunk of 0 reserves exactly what is asked for
+// (a list without room for padding): same-address atomics take about 1.8 ns
+// each, which is what sharing saves.
+__device__ __forceinline__ void chunk_take(u64* word, unsigned chunk, unsigned* ctr, unsigned total, unsigned& pos,
+                                           unsigned& avail, unsigned& fresh, DevState* st, unsigned cap) {
+  if (chunk == 0) {
+    pos = atomicAdd(ctr, total);
+    avail = total;
+    return;
+  }
+  for (;;) {
+    const u64 old = atomicAdd(word, (u64)total);
+    const unsigned used = (unsigned)old;
+    pos = (unsigned)(old >> 32) + used;
+    if (used + total <= chunk) {
+      avail = total;
+      return;
+    }
+    if (used <= chunk) {  // the one that overruns the chunk fetches the next
+      avail = chunk - used;
+      fresh = atomicAdd(ctr, chunk);
+      atomicExch(word, ((u64)fresh << 32) | (total - avail));
+      return;
+    }
+    for (unsigned spin = 0; (unsigned)*(volatile u64*)word > chunk; spin++)
+      if (spin > (1u << 24)) {  // seconds: the other warp is gone
+        atomicOr(&st->error, kErrTimeout);
+        avail = 0;
+        fresh = cap;  // nothing is written there
+        return;
+      }
+  }
+}
+
 struct BorSmem {
   unsigned cursor;                    // entries this CTA kept in the current offer pass
   int seg_n;                          // segments of the list read next (0 = dense)
@@ -65,11 +103,6 @@ struct BorSmem {
   unsigned base[2];
 };
 
-__device__ __forceinline__ int ld_ca(const int* p) {
-  int v;
-  asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ u64 ld_ca64(const u64* p) {
   u64 v;
   asm volatile("ld.global.ca.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -83,51 +116,70 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
 __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned* p, unsigned v) {
-  unsigned o;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(o) : "l"(p), "r"(v) : "memory");
-  return o;
+__device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Barrier among the first `active` CTAs of a cooperative launch. One release
-// add per CTA and an acquire poll of the generation word by one thread; the
-// other threads are ordered through the CTA barriers on both sides. The wait
-// is bounded (kErrTimeout, and every later barrier then returns false).
+// Barrier among the first `active` CTAs of a cooperative launch: one release
+// add per CTA to a counter that only grows, and an acquire poll of the same
+// counter by one thread; the other threads are ordered through the CTA
+// barriers on both sides. (A counter that the last CTA resets before it
+// releases a generation word took 1.85 us on 32 to 296 CTAs.) The wait is
+// bounded (kErrTimeout, and every later barrier then returns false).
 struct GridSync {
   static constexpr bool kGrid = true;
   DevState* st;
-  unsigned rank, active, gen;
-  __device__ __forceinline__ void init(DevState* s) {
+  unsigned* word;  // zero when the launch starts
+  unsigned rank, active, target;
+  __device__ __forceinline__ void init(DevState* s, unsigned* counter) {
     st = s;
+    word = counter;
     rank = blockIdx.x;
     active = gridDim.x;
-    gen = ld_volatile(&s->bar_gen);
+    target = 0;
+  }
+  __device__ __forceinline__ bool poll(const unsigned* p, unsigned at_least, bool nap) {
+    u64 t0 = 0;
+    for (unsigned spin = 1; (int)(ld_acquire_gpu(p) - at_least) < 0; spin++) {
+      if (nap) __nanosleep(100);
+      if ((spin & 1023u) == 0) {  // the limit, checked now and then
+        const u64 now = globaltimer_ns();
+        if (!t0) t0 = now;
+        if (now - t0 > kBarrierTimeoutNs) atomicOr(&st->error, kErrTimeout);
+        if (ld_volatile(&st->error) & kErrTimeout) return false;
+      }
+    }
+    return true;
   }
   __device__ __forceinline__ bool sync() {
     __syncthreads();
+    if (active == 1) return true;
+    target += active;
     bool ok = true;
     if (threadIdx.x == 0) {
-      const unsigned arrived = atom_add_acq_rel_gpu(&st->bar_count, 1u);
-      if (arrived == active - 1) {
-        st->bar_count = 0u;
-        st_release_gpu(&st->bar_gen, gen + 1u);
-      } else {
-        u64 t0 = 0;
-        for (unsigned spin = 1; ld_acquire_gpu(&st->bar_gen) == gen; spin++) {
-          if ((spin & 1023u) == 0) {  // the limit, checked now and then
-            const u64 now = globaltimer_ns();
-            if (!t0) t0 = now;
-            if (now - t0 > kBarrierTimeoutNs) atomicOr(&st->error, kErrTimeout);
-            if (ld_volatile(&st->error) & kErrTimeout) {
-              ok = false;
-              break;
-            }
-          }
-        }
+      red_add_release_gpu(word, 1u);
+      ok = poll(word, target, false);
+    }
+    return __syncthreads_and(ok);
+  }
+  // All CTAs of the launch again, after rounds some of them `left`: those wait
+  // until the first CTA, done with the rounds, opens gate number `gate`, and
+  // take over its count of the barriers.
+  __device__ __forceinline__ bool regroup(bool left, unsigned gate) {
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (rank == 0) {
+        st->gate_target = target;
+        st_release_gpu(&st->gate, gate);
+      } else if (left) {
+        ok = poll(&st->gate, gate, true);
       }
     }
-    gen++;
-    return __syncthreads_and(ok);
+    active = gridDim.x;
+    ok = __syncthreads_and(ok);
+    if (left) target = ld_volatile(&st->gate_target);
+    return ok;
   }
 };
 
@@ -135,9 +187,9 @@ struct GridSync {
 // over its first CTA alone.
 struct ClusterSync {
   static constexpr bool kGrid = false;
-  unsigned rank, active;
-  __device__ __forceinline__ void init(unsigned ctas) {
-    active = ctas;
+  unsigned rank, active, ctas;
+  __device__ __forceinline__ void init(unsigned n) {
+    active = ctas = n;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   }
   __device__ __forceinline__ bool sync() {
@@ -147,6 +199,11 @@ struct ClusterSync {
       asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     }
     return true;
+  }
+  // The whole cluster again: the CTAs that left the rounds wait at its barrier.
+  __device__ __forceinline__ bool regroup(bool, unsigned) {
+    active = ctas;
+    return sync();
   }
 };
 
@@ -316,6 +373,7 @@ __device__ __forceinline__ void bor_roots_step(const BorArgs& a, const int (&v)[
         }
       }
   }
+  if (!out) return;
   // CTA-wide reservation of the kept roots
   const unsigned cnt = __popc(keep);
   unsigned incl = cnt;
@@ -343,8 +401,16 @@ __device__ __forceinline__ void bor_roots_step(const BorArgs& a, const int (&v)[
 // Rounds from state `b` until the list is empty (true) or, grid-wide, until
 // it is at most a.tail entries long (false: `b` is where to go on). `fresh`:
 // the first list's endpoints are roots and differ. CTAs beyond what a round
-// needs leave for good; their `b` is meaningless.
-template <int T, int E, class Sync>
+// needs leave (`left`); their `b` is meaningless.
+//
+// Below some 10^5 entries a round is bound by its dependent L2 accesses (0.35
+// us a load or atomic) and barriers, so the loads that do not depend on each
+// other are issued together, the entries of a CTA with one tile stay in
+// registers from the offer to the mark pass (kKeep: not in k_round, whose 32
+// registers a thread they would spill, 2 % slower on RMAT-22), and where the vertices are few
+// for the threads at work the roots pass looks at all of them instead of
+// keeping a list.
+template <int T, int E, bool kKeep, class Sync>
 __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool fresh_list, Sync& sy, BorSmem& s,
                                            bool& left) {
   constexpr int N = 2 * E;
@@ -355,6 +421,15 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
   unsigned atomics = 0;
   const bool stamp = sy.rank == 0 && tid == 0;
   bool done = true;
+  // CTAs that work on a round of W entries, of `active`
+  auto wanted = [&](unsigned W, unsigned active) {
+    unsigned want = active;
+    if (Sync::kGrid && a.min_tiles > 0) want = min(want, max(1u, (W + a.min_tiles * tile - 1) / (a.min_tiles * tile)));
+    if ((!Sync::kGrid || !a.tail) && W <= a.solo) want = 1;
+    return want;
+  };
+  // whether a roots pass by `threads` threads looks at all vertices
+  auto scan_roots = [&](unsigned threads) { return (u64)(unsigned)a.nodes <= 4ull * threads; };
   while (b.W) {
     if (b.r >= ECL_MAX_ROUNDS) {
       if (stamp) atomicOr(&st->error, kErrRounds);
@@ -364,12 +439,7 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
       done = false;
       break;
     }
-    unsigned want = sy.active;
-    if (Sync::kGrid) {
-      if (a.min_tiles > 0) want = min(want, max(1u, (b.W + a.min_tiles * tile - 1) / (a.min_tiles * tile)));
-    } else if (b.W <= a.solo) {
-      want = 1;
-    }
+    const unsigned want = wanted(b.W, sy.active);
     if (want < sy.active) {
       sy.active = want;
       if (sy.rank >= want) {
@@ -383,10 +453,13 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     int4* out = (b.k & 1) ? a.wl0 : a.wl1;
     const unsigned W = b.W, ntiles = (W + tile - 1) / tile;
     const unsigned region = share_region(W, tile, start, stride);
+    const bool one = kKeep && ntiles <= stride;  // no CTA has a second tile
+    int4 e[E];
+    bool ok[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) ok[i] = false;
     // ---- offer
     for (unsigned t = start; t < ntiles; t += stride) {
-      int4 e[E];
-      bool ok[E];
 #pragma unroll
       for (int i = 0; i < E; i++) {
         const unsigned idx = t * tile + i * T + tid;
@@ -462,6 +535,25 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     }
     if (!sy.sync()) break;
     if (stamp) st->t_round[ph][2 * b.r] = globaltimer_ns();
+    u64 mx[E], my[E];
+    auto minima = [&]() {
+#pragma unroll
+      for (int i = 0; i < E; i++) {
+        mx[i] = ok[i] && e[i].x != b.skip ? ld_ca64(a.minv + e[i].x) : kNoEdge;
+        my[i] = ok[i] && e[i].y != b.skip ? ld_ca64(a.minv + e[i].y) : kNoEdge;
+      }
+    };
+    auto mark = [&]() {
+#pragma unroll
+      for (int i = 0; i < E; i++) {
+        const u64 key = edge_key(e[i].z, e[i].w);
+        if (ok[i] && (key == mx[i] || key == my[i])) {
+          cas_union(e[i].x, e[i].y, a.parent);
+          a.inMST[e[i].w] = 1;
+        }
+      }
+    };
+    if (one) minima();
     const unsigned W2 = ld_volatile(&st->wl_count[ph][b.r + 1]);
     b.r++;
     if (W2 == 0) {
@@ -470,43 +562,39 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     }
     // The next round's segment table is read here, two barriers before any CTA
     // can be at the end of that round's offer pass and publish new segments.
-    if (!fresh) bor_seg_load<T>(s, st, (int)stride);
+    if (!fresh) {
+      if (stride > 1) bor_seg_load<T>(s, st, (int)stride);
+      else if (tid == 0) s.seg_n = 0;  // one segment, from position 0
+    }
     // ---- mark: the first round's scan list, or this CTA's own segment
-    {
+    if (one) {
+      mark();
+    } else {
       const unsigned cnt = fresh ? W : s.cursor;
       const unsigned step = fresh ? stride * tile : tile;
       const int4* src = fresh ? in : out + region;
       for (unsigned base = fresh ? start * tile : 0u; base < cnt; base += step) {
-        int4 e[E];
-        u64 mx[E], my[E];
 #pragma unroll
         for (int i = 0; i < E; i++) {
           const unsigned idx = base + i * T + tid;
           e[i] = idx < cnt ? __ldcg(src + idx) : make_int4(-1, -1, 0, 0);
+          ok[i] = e[i].x >= 0;
         }
-#pragma unroll
-        for (int i = 0; i < E; i++) {
-          mx[i] = e[i].x >= 0 && e[i].x != b.skip ? ld_ca64(a.minv + e[i].x) : kNoEdge;
-          my[i] = e[i].x >= 0 && e[i].y != b.skip ? ld_ca64(a.minv + e[i].y) : kNoEdge;
-        }
-#pragma unroll
-        for (int i = 0; i < E; i++) {
-          const u64 key = edge_key(e[i].z, e[i].w);
-          if (e[i].x >= 0 && (key == mx[i] || key == my[i])) {
-            cas_union(e[i].x, e[i].y, a.parent);
-            a.inMST[e[i].w] = 1;
-          }
-        }
+        minima();
+        mark();
       }
     }
     if (!sy.sync()) break;
     // ---- roots
-    int* rout = (b.flips & 1) ? a.roots1 : a.roots0;
+    const bool all = scan_roots(stride * T) || (b.first && 4ull * W2 >= (unsigned)a.nodes);
+    // threads of the next roots pass, and whether it will want a list
+    const unsigned ahead = Sync::kGrid && W2 <= a.tail ? (W2 <= a.solo ? 1u : (unsigned)kTailCtas) * kTailThreads
+                                                       : wanted(W2, stride) * T;
+    int* rout = scan_roots(ahead) ? nullptr : ((b.flips & 1) ? a.roots1 : a.roots0);
     const int* rin = (b.flips & 1) ? a.roots0 : a.roots1;
     unsigned* rctr = &st->root_cnt[ph][b.flips % 3];
     int flip = 0;
     constexpr int U = E > 1 ? 4 : 2;
-    const bool all = b.first && 4ull * W2 >= (unsigned)a.nodes;
     if (b.first && !all) {  // few entries for the vertices: take the roots from this CTA's entries
       const unsigned cnt = fresh ? W : s.cursor;
       const unsigned step = fresh ? stride * T : T;
@@ -514,9 +602,9 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
       // every CTA thread takes every step (the step synchronises the CTA)
       for (unsigned base = fresh ? start * T : 0u; base < cnt; base += step, flip ^= 1) {
         const unsigned idx = base + tid;
-        const int4 e = idx < cnt ? __ldcg(src + idx) : make_int4(-1, -1, 0, 0);
-        const int v[2] = {e.x, e.y};
-        const bool valid[2] = {e.x >= 0, e.x >= 0};
+        const int4 x = idx < cnt ? __ldcg(src + idx) : make_int4(-1, -1, 0, 0);
+        const int v[2] = {x.x, x.y};
+        const bool valid[2] = {x.x >= 0, x.x >= 0};
         bor_roots_step<2>(a, v, valid, true, b.skip, rout, rctr, flip, s);
       }
       if (b.skip >= 0 && start == 0) {  // `skip` is in no slot: carried by hand
@@ -542,11 +630,11 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     if (tid == 0) s.cursor = 0;
     if (!sy.sync()) break;
     if (stamp) st->t_round[ph][2 * b.r - 1] = globaltimer_ns();
-    b.C = ld_volatile(rctr);
+    if (rout) b.C = ld_volatile(rctr);
     b.flips++;
     if (b.skip >= 0) b.skip = ld_ca(a.parent + b.skip);
     if (!fresh) {
-      b.nseg = (int)stride;
+      b.nseg = stride > 1 ? (int)stride : 0;
       b.k++;
     }
     b.first = 0;
@@ -568,13 +656,13 @@ __global__ void __launch_bounds__(kBorThreads, kBorBlocks) k_round(BorArgs a) {
   b.first = 1;
   b.skip = a.phase == 1 ? st->giant : -1;
   GridSync sy;
-  sy.init(st);
+  sy.init(st, &st->bar[a.phase]);
   bor_smem_init(s);
   __syncthreads();
   const bool stamp = sy.rank == 0 && threadIdx.x == 0;
   if (stamp) st->t_round_start[a.phase] = globaltimer_ns();
   bool left;
-  const bool done = bor_rounds<kBorThreads, kBorEpt>(a, b, true, sy, s, left);
+  const bool done = bor_rounds<kBorThreads, kBorEpt, false>(a, b, true, sy, s, left);
   if (stamp && !left) {
     st->rounds[a.phase] = b.r;
     if (done) b.W = 0;
@@ -602,7 +690,7 @@ __global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads
       bor_seg_load<kTailThreads>(s, st, b.nseg);
       __syncthreads();
     }
-    bor_rounds<kTailThreads, kTailEpt>(a, b, true, sy, s, left);
+    bor_rounds<kTailThreads, kTailEpt, true>(a, b, true, sy, s, left);
     if (sy.rank == 0 && threadIdx.x == 0 && !left) st->rounds[a.phase] = b.r;
   }
   if (a.phase == 0 && st->filtered && sy.rank == 0) {
