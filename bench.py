@@ -797,10 +797,9 @@ def main():
                             "copy in overlaps the previous solve and copy back), wall clock over the steps",
                     "sync": {"value": world * g.edges / e2e_sync / 1e9, "ms": e2e_sync * 1e3,
                              "what": "one blocking ecl_mst_ctx_run_host call per step"}},
-            # per solve: k_prep, k_fill_chunks, k_fill_carry, k_scan x2, k_round x2, k_round_tail x2, k_flatten; the
-            # learned schedule adds k_sample and k_mlp_apply and launches all three light-scan
-            # variants (the two its split does not select exit at once; the heavy scan is one)
-            "gpu_launches": (14 if args.mode == "learned" else 10) * args.steps,
+            # per solve: k_prep, k_scan_light, k_round and k_round_tail, k_flatten and the two for the second
+            # light list, k_flatten, k_scan_heavy and the two; the learned schedule adds k_sample and k_mlp_apply
+            "gpu_launches": (13 if args.mode == "learned" else 11) * args.steps,
             "ablation": ablation,
             "heuristic_schedule": ({"value": world * g.edges / (np.mean(heur_ms) * 1e-3) / 1e9,
                                     "ms": float(np.mean(heur_ms)),

@@ -86,11 +86,8 @@ struct ClMem {
   }
   // Adds `x` to the same shared-memory counter of every CTA (one thread).
   __device__ __forceinline__ void add_all(unsigned* counter, unsigned x) const {
-    if (kOne) {
-      *counter += x;
-      return;
-    }
-    for (unsigned r = 0; r < (1u << log); r++) {
+    if (kOne) *counter += x;
+    else for (unsigned r = 0; r < (1u << log); r++) {
       unsigned a;
       asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(counter)), "r"(r));
       asm volatile("red.shared::cluster.add.u32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
@@ -221,7 +218,8 @@ __device__ void cl_rounds(const ClArgs& g, const ClMem<kOne>& M, ClusterSync& sy
   pass_no++;
   if (stamp) {
     st->wl_count[phase][0] = W;
-    st->scan_kept[phase] = W;
+    st->wl_kept[phase][0] = W;
+    st->lists[phase == 0 ? kListLight0 : kListHeavy].kept = W;
   }
   int r = 0;
   for (; W; r++) {

@@ -14,9 +14,9 @@
 #include "internal.h"
 #include "mst_device.cuh"
 #include "rounds_device.cuh"
+#include "scan_device.cuh"
 #include "group_device.cuh"
 #include "cluster_device.cuh"
-#include <functional>
 #include <vector>
 
 // Learned threshold/split (learned.cu). ecl_learned_sample uploads changed
@@ -24,7 +24,7 @@
 // features from it and from k_prep's degree statistics and runs the trained
 // MLP, writing DevState::threshold, filtered, quantile and split.
 int ecl_learned_sample(ecl_mst_ctx* c, const ecl_graph* d_graph, cudaStream_t s);
-int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* d_graph, cudaStream_t s, void* st);
+int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* d_graph, cudaStream_t s, void* st, int lists);
 int ecl_learned_upload(ecl_mst_ctx* c, cudaStream_t s);
 unsigned ecl_learned_weights_version();
 
@@ -52,12 +52,9 @@ struct ecl_mst_ctx {
   int sm_count = 0;
   int64_t max_nodes = 0, max_edges = 0;
   cudaStream_t stream = nullptr;
-  // the learned schedule's sample sort and MLP run on `side`, beside k_prep
-  // and the fill scan; the scan variants its split does not select run on
-  // `side` and `side2`, beside the selected one
-  cudaStream_t side = nullptr, side2 = nullptr;
+  // the learned schedule's sample sort (beside k_prep) and MLP run on `side`
+  cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr, prep_done = nullptr;
-  cudaEvent_t scan_fork = nullptr, scan_join[2] = {nullptr, nullptr};
   // the last solve's key, and the captured solve (CUDA graph) with its key
   std::vector<long long> last_key, exec_key;
   cudaGraphExec_t exec = nullptr;
@@ -110,7 +107,8 @@ struct ecl_mst_ctx {
   std::vector<AsyncCall> async_calls;
   int* slist = nullptr;    // ECL_FLAG_NO_TUPLES: vertex of every CSR entry (allocated on first use)
   int vertex_grid = 0;     // ECL_FLAG_NO_EDGE_BASED: cooperative grid of the vertex-centric rounds
-  int* first_v = nullptr;  // tile -> vertex table of the edge-balanced scans
+  int* first_v = nullptr;  // task -> row table of the scans
+  unsigned* tree_bits = nullptr;  // bit v: v lies in the light phase's largest tree
   int first_v_cap = 0;
   DevState* st = nullptr;
   DevState* st_host = nullptr;  // pinned
@@ -229,39 +227,17 @@ int launch_cluster(void (*kernel)(KArgs...), int size, int clusters, int threads
 
 int prepare_scan_kernels();
 int prepare_cluster_kernels();
+int prepare_round_kernels();
 
-// Entries of the tile->vertex table buffer for up to `edges` CSR entries: the
-// table (tiles + 1) and the fill scan's chunk maxima.
-int64_t first_v_entries(int64_t edges) {
-  const int64_t tiles = edges / kGran + 1;
-  return tiles + 1 + tiles / kFillChunk + 1;
-}
+// Bytes of the vertex bits for up to `nodes` vertices.
+constexpr size_t tree_bits_bytes(int64_t nodes) { return (size_t)(nodes + 31) / 32 * sizeof(unsigned); }
 
-// k_prep, then the fill scan that completes the tile->vertex table
-// (first_v: pa.tiles + 1 entries, then room for the chunk maxima).
-// k_prep, then the max scan of the tile->vertex table. `after_prep`, when
-// given, is enqueued between the two (the learned schedule forks its MLP off
-// there, once k_prep's degree statistics are complete).
-int enqueue_prep(const PrepArgs& pa, int sm_count, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr,
-                 const std::function<int()>& after_prep = nullptr) {
-  ECL_CUDA_TRY(cudaMemsetAsync(pa.first_v, 0, sizeof(int) * (size_t)pa.tiles, s));
-  const int prep_grid = (int)std::min<int64_t>((pa.nodes + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
-  if (win) {
-    int st = launch_ex(k_prep, std::max(prep_grid, 1), kThreads, 0, s, false, win, pa);
-    if (st) return st;
-  } else {
-    k_prep<<<std::max(prep_grid, 1), kThreads, 0, s>>>(pa);
-  }
-  ECL_CUDA_TRY(cudaGetLastError());
-  if (after_prep) {
-    const int st = after_prep();
-    if (st) return st;
-  }
-  const int chunks = (pa.tiles + kFillChunk - 1) / kFillChunk;
-  int* chunk_max = pa.first_v + pa.tiles + 1;
-  k_fill_chunks<<<chunks, 1024, 0, s>>>(pa.first_v, pa.tiles, chunk_max);
-  k_fill_carry<<<chunks, 1024, 0, s>>>(pa.first_v, pa.tiles, chunk_max, pa.nodes);
-  return cuda_status(cudaGetLastError());
+// Entries of the task->row table for up to `edges` CSR entries.
+int64_t first_v_entries(int64_t edges) { return edges / kGran + 2; }
+
+int enqueue_prep(const PrepArgs& pa, int sm_count, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr) {
+  const int grid = (int)std::min<int64_t>((pa.nodes + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
+  return launch_ex(k_prep, std::max(grid, 1), kThreads, 0, s, false, win, pa);
 }
 
 // Round-kernel ablation bits from the option flags.
@@ -335,10 +311,6 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)))) return fail(st);
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming)))) return fail(st);
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->prep_done, cudaEventDisableTiming)))) return fail(st);
-  if ((st = cuda_status(cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking)))) return fail(st);
-  if ((st = cuda_status(cudaEventCreateWithFlags(&c->scan_fork, cudaEventDisableTiming)))) return fail(st);
-  for (auto& e : c->scan_join)
-    if ((st = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)))) return fail(st);
   const size_t slot_bytes = (size_t)max_nodes * (2 * sizeof(u64) + sizeof(int));
   if ((st = cuda_status(cudaMalloc(&c->slots, slot_bytes)))) return fail(st);
   c->l2_persist_max = prop.persistingL2CacheMaxSize > 0 ? (size_t)prop.persistingL2CacheMaxSize : 0;
@@ -346,6 +318,7 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   if ((st = alloc_worklists(c, false))) return fail(st);
   c->first_v_cap = (int)first_v_entries(max_edges);
   if ((st = cuda_status(cudaMalloc(&c->first_v, (size_t)c->first_v_cap * sizeof(int))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->tree_bits, tree_bits_bytes(max_nodes))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->st, sizeof(DevState))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->ml_params, ECL_MLP_PARAMS * sizeof(float))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->ml_feat, ECL_MLP_INPUTS * sizeof(float))))) return fail(st);
@@ -361,6 +334,7 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   c->group_grid = coop_grid((const void*)k_group, kGroupThreads, c->sm_count);
   c->vertex_grid = coop_grid((const void*)k_rounds_vertex, kRoundThreads, c->sm_count);
   if ((st = prepare_scan_kernels())) return fail(st);
+  if ((st = prepare_round_kernels())) return fail(st);
   if ((st = prepare_cluster_kernels())) return fail(st);
   if (c->round_grid <= 0 || c->abl_grid <= 0 || c->group_grid <= 0 || c->vertex_grid <= 0) return fail(ECL_ERR_CUDA);
   *out = c;
@@ -379,6 +353,7 @@ extern "C" void ecl_mst_ctx_destroy(ecl_mst_ctx* c) {
   cudaFree(c->wl[0]);
   cudaFree(c->wl[1]);
   cudaFree(c->first_v);
+  cudaFree(c->tree_bits);
   cudaFree(c->slist);
   cudaFree(c->ml_params);
   cudaFree(c->ml_feat);
@@ -405,15 +380,10 @@ extern "C" void ecl_mst_ctx_destroy(ecl_mst_ctx* c) {
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   if (c->side) cudaStreamSynchronize(c->side);
-  if (c->side2) cudaStreamSynchronize(c->side2);
   if (c->exec) cudaGraphExecDestroy(c->exec);
   if (c->fork) cudaEventDestroy(c->fork);
   if (c->join) cudaEventDestroy(c->join);
   if (c->prep_done) cudaEventDestroy(c->prep_done);
-  if (c->scan_fork) cudaEventDestroy(c->scan_fork);
-  for (cudaEvent_t e : c->scan_join)
-    if (e) cudaEventDestroy(e);
-  if (c->side2) cudaStreamDestroy(c->side2);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -469,72 +439,59 @@ extern "C" int ecl_mst_ctx_sync(ecl_mst_ctx* c) {
 
 namespace {
 
-// Opt the scan variants into their dynamic shared memory (once per device).
+// Opt the scans into their shared memory (once per device).
 int prepare_scan_kernels() {
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kLight, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<4>()));
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kLight, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<8>()));
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kLight, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<16>()));
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kHeavy, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<4>()));
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kHeavy, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<8>()));
-  ECL_CUDA_TRY(cudaFuncSetAttribute(k_scan<kHeavy, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem_bytes<16>()));
+  for (auto k : {k_scan_light<false>, k_scan_light<true>})
+    ECL_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem<true>)));
+  for (auto k : {k_scan_heavy<false>, k_scan_heavy<true>})
+    ECL_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem<false>)));
   return ECL_OK;
 }
 
-// Persistent scan: exactly as many CTAs as can be resident at once (a CTA
-// started late would finish its share late), each looping over tiles. The
-// warps' slot chunk is sized so that the unused chunk tails (at most
-// chunk - 1 per warp) fit in the worklist's slack.
-template <int KIND, int EPT>
-int launch_scan_ept(const ScanArgs& sa, cudaStream_t s, const cudaAccessPolicyWindow* win) {
-  const int64_t m = sa.edges;
-  const int64_t tile = ScanCfg<EPT>::kTile;
-  const int tiles = (int)((m + tile - 1) / tile);
-  int per_sm = 0;
-  ECL_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan<KIND, EPT>, kScanThreads,
-                                                             scan_smem_bytes<EPT>()));
-  int blocks = std::max(1, std::min(tiles, std::max(1, per_sm) * sa.sm_count));
+// Shared memory an SM sets aside while the rounds and the kernels between the
+// scans run, in per cent. An SM changes the split between shared memory and L1
+// only when it is idle, so with several streams a kernel of the smallest
+// split waits for the SMs that run another's scan (3 x 72 KB) to drain: a
+// batch of 39 large graphs on 8 streams 8.0 ms at 25 to 60 per cent, 9.1 with
+// the driver's choice; one solve at a time is the same (RMAT-22 1.47 ms) but at
+// 12 or 100, where k_round's CTAs or its L1 hits go missing (1.57, 1.83).
+constexpr int kCarveout = 40;
+int prepare_round_kernels() {
+  for (const void* k : {(const void*)k_round, (const void*)k_round_tail, (const void*)k_prep, (const void*)k_flatten,
+                        (const void*)k_group})
+    ECL_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout));
+  return ECL_OK;
+}
+
+// Persistent scan: as many CTAs as can be resident at once, or one per
+// kScanWarps tasks. The CTAs' slot chunk is sized so that the unused chunk
+// tails (at most chunk - 1 per CTA and list, two lists to an array) fit in the
+// worklist's slack; 0 = slots are reserved exactly.
+int launch_scan(int kind, const ScanArgs& sa, int sm_count, unsigned wl_slack, cudaStream_t s,
+                const cudaAccessPolicyWindow* win = nullptr) {
+  const int blocks = std::max(1, std::min((sa.tiles + kScanWarps - 1) / kScanWarps, kScanBlocks * sm_count));
   ScanArgs a = sa;
-  const int64_t warps = (int64_t)blocks * kScanWarps;
-  a.chunk = (unsigned)std::max<int64_t>(1, std::min<int64_t>(kScanMaxChunk, (int64_t)sa.wl_slack / warps));
-  if (win) return launch_ex(k_scan<KIND, EPT>, blocks, kScanThreads, scan_smem_bytes<EPT>(), s, false, win, a);
-  k_scan<KIND, EPT><<<blocks, kScanThreads, scan_smem_bytes<EPT>(), s>>>(a);
-  return cuda_status(cudaGetLastError());
+  a.chunk = std::min(kScanMaxChunk, wl_slack / (unsigned)(2 * blocks));
+  if (a.chunk < kScanMinChunk) a.chunk = 0;
+  const bool vec = (((uintptr_t)(kind == kLight ? sa.eweight : sa.nlist)) & 15) == 0;
+  if (kind == kLight)
+    return launch_ex(vec ? k_scan_light<true> : k_scan_light<false>, blocks, kScanThreads, sizeof(ScanSmem<true>), s,
+                     false, win, a);
+  return launch_ex(vec ? k_scan_heavy<true> : k_scan_heavy<false>, blocks, kScanThreads, sizeof(ScanSmem<false>), s,
+                   false, win, a);
 }
 
-template <int KIND>
-int launch_scan(int ept, const ScanArgs& sa, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr) {
-  if (ept == 4) return launch_scan_ept<KIND, 4>(sa, s, win);
-  if (ept == 8) return launch_scan_ept<KIND, 8>(sa, s, win);
-  return launch_scan_ept<KIND, 16>(sa, s, win);
-}
-
-// Scan variants to launch: the one the split selects, or all three (each
-// exits unless st->split selects it) when the split is chosen on the device.
-// Those three go on forked streams, so the two that exit at once do so beside
-// the selected one instead of after it.
-template <int KIND>
-int launch_scans(ecl_mst_ctx* c, bool device_split, int split, const ScanArgs& sa, cudaStream_t s,
-                 const cudaAccessPolicyWindow* win) {
-  if (KIND == kHeavy && ECL_HEAVY_EPT) return launch_scan<KIND>(ECL_HEAVY_EPT, sa, s, win);
-  if (!device_split) return launch_scan<KIND>(scan_ept(split), sa, s, win);
-  const cudaStream_t br[2] = {c->side, c->side2};
-  ECL_CUDA_TRY(cudaEventRecord(c->scan_fork, s));
-  for (cudaStream_t b : br) ECL_CUDA_TRY(cudaStreamWaitEvent(b, c->scan_fork, 0));
-  int st;
-  if ((st = launch_scan<KIND>(8, sa, s, win))) return st;  // the split the network picks most often
-  if ((st = launch_scan<KIND>(4, sa, br[0], win))) return st;
-  if ((st = launch_scan<KIND>(16, sa, br[1], win))) return st;
-  for (int i = 0; i < 2; i++) {
-    ECL_CUDA_TRY(cudaEventRecord(c->scan_join[i], br[i]));
-    ECL_CUDA_TRY(cudaStreamWaitEvent(s, c->scan_join[i], 0));
-  }
-  return ECL_OK;
+// Flattened parent[] and the largest tree's vertex bits.
+int launch_flatten(int list, int* parent, int n, const DevState* st, unsigned* tree_bits, int sm_count, cudaStream_t s,
+                   const cudaAccessPolicyWindow* win = nullptr) {
+  const int grid = (int)std::min<int64_t>(((int64_t)n + 4 * kThreads - 1) / (4 * kThreads), (int64_t)sm_count * 4);
+  return launch_ex(k_flatten, std::max(grid, 1), kThreads, 0, s, false, win, parent, n, st, tree_bits, list);
 }
 
 // One phase's Boruvka rounds: the grid-wide kernel, then the cluster kernel
 // that ends the phase. The ablation switches run the variants kept in
 // k_rounds. `per_sm`: the caller's limit on CTAs per SM (0 = none).
-int enqueue_rounds(const RoundArgs& ra, int edges, int sm_count, int per_sm, int round_grid, int abl_grid,
+int enqueue_rounds(const RoundArgs& ra, int list, int edges, int sm_count, int per_sm, int round_grid, int abl_grid,
                    cudaStream_t s, const cudaAccessPolicyWindow* win) {
   const int limit = per_sm > 0 ? per_sm * sm_count : INT_MAX;
   if (ra.abl) {
@@ -545,7 +502,7 @@ int enqueue_rounds(const RoundArgs& ra, int edges, int sm_count, int per_sm, int
   BorArgs ba{};
   ba.phase = ra.phase;
   ba.nodes = ra.nodes;
-  ba.list = ra.wl0;
+  ba.list = list;
   ba.wl0 = ra.wl0;
   ba.wl1 = ra.wl1;
   ba.wl_cap = ra.wl_cap;
@@ -643,7 +600,7 @@ bool l2_window(const ecl_mst_ctx* c, const Slots& sl, bool parent_only, cudaAcce
 // The learned schedule's steps around k_prep. The weight sample is sorted on
 // `side` from the start of the solve (ecl_learned_sample); k_prep gathers the
 // degree statistics into `acc` on the solve's stream; the MLP then runs on
-// `side` beside the fill scan, and the light scan waits for it.
+// `side`, and the light scan waits for it.
 struct LearnedPlan {
   cudaStream_t side;
   cudaEvent_t prep_done, join;
@@ -662,11 +619,19 @@ int learned_fork(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t q, LearnedPlan
   return ecl_learned_sample(c, g, lp->side);
 }
 
+// The share of the entries that the light phase will take, as far as the host
+// can tell: the reference heuristic's expectation where the threshold is
+// chosen on the device.
+double light_share(const mst_opts* o, int n, int m) {
+  if (o->threshold_mode == ECL_THRESH_NONE) return 1.0;
+  if (o->threshold_mode == ECL_THRESH_QUANTILE) return std::min(1.0, (double)o->quantile);
+  return m / n < 4 ? 1.0 : (std::min(19, (int)(3.0 * n * 20 / m)) + 1) / 21.0;
+}
+
 int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, const mst_opts* o,
                   cudaStream_t s, bool timed, const LearnedPlan* lp = nullptr) {
   const int n = g->nodes, m = g->edges;
   const int split = o->degree_split > 0 ? o->degree_split : kDefaultSplit;
-  const bool device_split = o->threshold_mode == ECL_THRESH_LEARNED;
   const int tiles = (int)(((int64_t)m + kGran - 1) / kGran);
   const Slots sl = slots_for(c->slots, n);
   // L2 persistence: k_prep writes the slots and parent, the rounds hammer
@@ -739,19 +704,28 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   pa.quantile = o->quantile;
   pa.st = c->st;
   pa.feat = lp ? lp->acc : nullptr;
+  const unsigned abl = round_ablation(o->flags);
+  pa.both_slots = abl != 0;
+  // The launches that lists split by weight need (split_ranks): about 20 us if
+  // the device then splits none. Below six entries per vertex it does not pay (a
+  // 1500 x 2000 grid 0.94 ms against 0.82), and the ablation variants keep one
+  // list per phase.
+  const bool lists = abl == 0 && !(o->flags & ECL_FLAG_NO_EDGE_BASED) && m / n >= 6 &&
+                     (n >= kMidNodes || light_share(o, n, m) * 0.5 * m >= kSplitMin);
+  pa.use_lists = lists;
+  // whether the heavy phase can run at all (the device may still decide not)
+  const bool two_phases = o->threshold_mode == ECL_THRESH_LEARNED || o->threshold_mode == ECL_THRESH_EXPLICIT ||
+                          (o->threshold_mode == ECL_THRESH_QUANTILE && o->quantile < 1.0f) ||
+                          (o->threshold_mode == ECL_THRESH_HEURISTIC && m / n >= 4);
   int st;
-  std::function<int()> fork_mlp;
-  if (lp)
-    fork_mlp = [&]() -> int {
-      ECL_CUDA_TRY(cudaEventRecord(lp->prep_done, s));
-      ECL_CUDA_TRY(cudaStreamWaitEvent(lp->side, lp->prep_done, 0));
-      const int r = ecl_learned_apply(c, g, lp->side, c->st);
-      if (r) return r;
-      ECL_CUDA_TRY(cudaEventRecord(lp->join, lp->side));
-      return ECL_OK;
-    };
-  if ((st = enqueue_prep(pa, c->sm_count, s, win_all, fork_mlp))) return st;
-  if (lp) ECL_CUDA_TRY(cudaStreamWaitEvent(s, lp->join, 0));
+  if ((st = enqueue_prep(pa, c->sm_count, s, win_all))) return st;
+  if (lp) {  // the network, once k_prep's degree statistics are complete
+    ECL_CUDA_TRY(cudaEventRecord(lp->prep_done, s));
+    ECL_CUDA_TRY(cudaStreamWaitEvent(lp->side, lp->prep_done, 0));
+    if ((st = ecl_learned_apply(c, g, lp->side, c->st, lists))) return st;
+    ECL_CUDA_TRY(cudaEventRecord(lp->join, lp->side));
+    ECL_CUDA_TRY(cudaStreamWaitEvent(s, lp->join, 0));
+  }
   const bool no_tuples = (o->flags & (ECL_FLAG_NO_TUPLES | ECL_FLAG_NO_EDGE_BASED)) == ECL_FLAG_NO_TUPLES;
   if (no_tuples) {  // the vertex of every entry, for the gathers of the rounds
     const int sgrid = (int)std::min<int64_t>(((int64_t)m + kThreads - 1) / kThreads, (int64_t)c->sm_count * 16);
@@ -767,16 +741,16 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   sa.first_v = c->first_v;
   sa.tiles = tiles;
   sa.parent = sl.parent;
-  sa.wl = c->wl[0];
+  sa.wl0 = c->wl[0];
+  sa.wl1 = c->wl[1];
   sa.wl_cap = c->wl_cap;
+  sa.tree_bits = c->tree_bits;
   // a scan keeps at most m entries, m / 2 for the symmetric input the
   // half-size lists assume (more overflows, and the solve is repeated)
-  sa.wl_slack = c->wl_cap - (unsigned)(c->wl_full ? m : m / 2);
+  const unsigned wl_slack = c->wl_cap - (unsigned)(c->wl_full ? m : m / 2);
   sa.inMST = d_inMST;
-  sa.vec_ok = ((((uintptr_t)g->nlist) | ((uintptr_t)g->eweight)) & 15) == 0;
   sa.zero_vec = (((uintptr_t)d_inMST) & 15) == 0;
   sa.st = c->st;
-  sa.sm_count = c->sm_count;
   sa.ids = no_tuples ? 1 : 0;
   RoundArgs ra{};
   ra.nodes = n;
@@ -791,7 +765,7 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
   ra.small_tail = o->small_tail < 0 ? 0u : (o->small_tail == 0 ? kDefaultSmallTail : (unsigned)o->small_tail);
   if (o->flags & ECL_FLAG_NO_SMALL_TAIL) ra.small_tail = 0;
   ra.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
-  ra.abl = round_ablation(o->flags);
+  ra.abl = abl;
   ra.nlist = g->nlist;
   ra.eweight = g->eweight;
   ra.slist = c->slist;
@@ -819,25 +793,30 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
     return ECL_OK;
   }
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[5], s));
-  if ((st = launch_scans<kLight>(c, device_split, split, sa, s, nullptr))) return st;
+  if ((st = launch_scan(kLight, sa, c->sm_count, wl_slack, s))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   ra.phase = 0;
-  if ((st = enqueue_rounds(ra, m, c->sm_count, o->ctas_per_sm, c->round_grid, c->abl_grid, s, win_all))) return st;
+  auto rounds = [&](int list) {
+    return enqueue_rounds(ra, list, m, c->sm_count, o->ctas_per_sm, c->round_grid, c->abl_grid, s, win_all);
+  };
+  auto flatten = [&](int list) {
+    return launch_flatten(list, sl.parent, n, c->st, c->tree_bits, c->sm_count, s, win_par);
+  };
+  if ((st = rounds(kListLight0))) return st;
+  if (lists && ((st = flatten(kListLight1)) || (st = rounds(kListLight1)))) return st;
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-  const int fgrid = (int)std::min<int64_t>(((int64_t)n + kThreads - 1) / kThreads, (int64_t)c->sm_count * 16);
-  if (win_par) {
-    if ((st = launch_ex(k_flatten, std::max(fgrid, 1), kThreads, 0, s, false, win_par, sl.parent, n,
-                        (const DevState*)c->st)))
-      return st;
-  } else {
-    k_flatten<<<std::max(fgrid, 1), kThreads, 0, s>>>(sl.parent, n, c->st);
-    ECL_CUDA_TRY(cudaGetLastError());
-  }
-  if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[6], s));
-  if ((st = launch_scans<kHeavy>(c, device_split, split, sa, s, win_par))) return st;
-  if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[3], s));
   ra.phase = 1;
-  if ((st = enqueue_rounds(ra, m, c->sm_count, o->ctas_per_sm, c->round_grid, c->abl_grid, s, win_all))) return st;
+  if (two_phases) {
+    if (lists && n >= kMidNodes && ((st = flatten(kListMid)) || (st = rounds(kListMid)))) return st;
+    if ((st = flatten(kListHeavy))) return st;
+    if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[6], s));
+    if ((st = launch_scan(kHeavy, sa, c->sm_count, wl_slack, s, win_par))) return st;
+    if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+    if ((st = rounds(kListHeavy))) return st;
+  } else if (timed) {
+    ECL_CUDA_TRY(cudaEventRecord(c->ev[6], s));
+    ECL_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+  }
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[4], s));
   return ECL_OK;
 }
@@ -854,10 +833,10 @@ int fill_stats(ecl_mst_ctx* c, ecl_mst_stats* stats, bool timed, bool breakdown 
   stats->rounds[1] = h.rounds[1];
   stats->status = (int32_t)h.error;
   for (int p = 0; p < 2; p++) {
-    stats->scan_kept[p] = h.scan_kept[p];
+    stats->scan_kept[p] = (int64_t)h.lists[2 * p].kept + h.lists[2 * p + 1].kept;
     for (int r = 0; r < ECL_MAX_ROUNDS; r++) {
       stats->wl_in[p][r] = h.wl_count[p][r];
-      stats->wl_real[p][r] = r == 0 ? h.scan_kept[p] : h.wl_kept[p][r];
+      stats->wl_real[p][r] = h.wl_kept[p][r];
     }
   }
   stats->atomics = (int64_t)h.atomics;
@@ -1259,8 +1238,7 @@ namespace {
 constexpr int64_t kNaMaxNodes = 1 << 18;              // 262,144 vertices
 constexpr int64_t kNaMaxEdges = 1 << 20;              // 1,048,576 directed CSR entries
 constexpr int64_t kNaWlCap = kNaMaxEdges / 2;         // one-direction entries per worklist
-// tile -> vertex table entries, with the fill scan's chunk maxima
-constexpr int64_t kNaTiles = kNaMaxEdges / kGran + 2 + (kNaMaxEdges / kGran + 1) / kFillChunk + 1;
+constexpr int64_t kNaTiles = kNaMaxEdges / kGran + 2;  // task -> row table entries
 
 constexpr size_t na_align(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kNaOffState = 0;
@@ -1268,7 +1246,8 @@ constexpr size_t kNaOffMinv0 = na_align(kNaOffState + sizeof(DevState));
 constexpr size_t kNaOffMinv1 = na_align(kNaOffMinv0 + sizeof(u64) * kNaMaxNodes);
 constexpr size_t kNaOffParent = na_align(kNaOffMinv1 + sizeof(u64) * kNaMaxNodes);
 constexpr size_t kNaOffFirstV = na_align(kNaOffParent + sizeof(int) * kNaMaxNodes);
-constexpr size_t kNaOffWl0 = na_align(kNaOffFirstV + sizeof(int) * kNaTiles);
+constexpr size_t kNaOffBits = na_align(kNaOffFirstV + sizeof(int) * kNaTiles);
+constexpr size_t kNaOffWl0 = na_align(kNaOffBits + tree_bits_bytes(kNaMaxNodes));
 constexpr size_t kNaOffWl1 = na_align(kNaOffWl0 + sizeof(int4) * kNaWlCap);
 constexpr size_t kNaBytes = na_align(kNaOffWl1 + sizeof(int4) * kNaWlCap);  // about 21 MB
 
@@ -1307,7 +1286,7 @@ int na_setup(int dev, NaDevice** out) {
     d.abl_grid = std::min(coop_grid((const void*)k_rounds, kRoundThreads, d.sm_count), kMaxRoundCtas);
     d.group_grid = coop_grid((const void*)k_group, kGroupThreads, d.sm_count);
     int ps = prepare_scan_kernels();
-    if (ps || (ps = prepare_cluster_kernels())) return ps;
+    if (ps || (ps = prepare_round_kernels()) || (ps = prepare_cluster_kernels())) return ps;
     if (d.round_grid <= 0 || d.abl_grid <= 0 || d.group_grid <= 0) return ECL_ERR_CUDA;
     d.ready = true;
   }
@@ -1413,9 +1392,9 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   pa.explicit_thr = o.threshold;
   pa.split = split;
   pa.quantile = o.quantile;
+  pa.both_slots = round_ablation(o.flags) != 0;
   pa.st = dst;
-  st = enqueue_prep(pa, d->sm_count, s);
-  if (st) return st;
+  if ((st = enqueue_prep(pa, d->sm_count, s))) return st;
   ScanArgs sa{};
   sa.nodes = n;
   sa.edges = m;
@@ -1425,15 +1404,15 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   sa.first_v = first_v;
   sa.tiles = tiles;
   sa.parent = parent;
-  sa.wl = wl0;
+  sa.wl0 = wl0;
+  sa.wl1 = wl1;
   sa.wl_cap = (unsigned)kNaWlCap;
+  sa.tree_bits = (const unsigned*)(d->base + kNaOffBits);
   // within the stated limit a scan keeps at most m / 2 entries
-  sa.wl_slack = (unsigned)std::max<int64_t>(0, kNaWlCap - m / 2);
+  const unsigned wl_slack = (unsigned)std::max<int64_t>(0, kNaWlCap - m / 2);
   sa.inMST = d_inMST;
-  sa.vec_ok = ((((uintptr_t)g->nlist) | ((uintptr_t)g->eweight)) & 15) == 0;
   sa.zero_vec = (((uintptr_t)d_inMST) & 15) == 0;
   sa.st = dst;
-  sa.sm_count = d->sm_count;
   RoundArgs ra{};
   ra.nodes = n;
   ra.wl0 = wl0;
@@ -1449,15 +1428,13 @@ extern "C" int ecl_mst_run_device_noalloc(const ecl_graph* g, uint8_t* d_inMST,
   ra.count_atomics = (o.flags & ECL_FLAG_STATS) ? 1 : 0;
   ra.abl = round_ablation(o.flags);
   ra.min_tiles = kDefaultMinTiles;
-  if ((st = launch_scan<kLight>(scan_ept(split), sa, s))) return st;
+  if ((st = launch_scan(kLight, sa, d->sm_count, wl_slack, s))) return st;
   ra.phase = 0;
-  if ((st = enqueue_rounds(ra, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
-  const int fgrid = (int)std::min<int64_t>(((int64_t)n + kThreads - 1) / kThreads, (int64_t)d->sm_count * 16);
-  k_flatten<<<std::max(fgrid, 1), kThreads, 0, s>>>(parent, n, dst);
-  ECL_CUDA_TRY(cudaGetLastError());
-  if ((st = launch_scan<kHeavy>(heavy_ept(split), sa, s))) return st;
+  if ((st = enqueue_rounds(ra, kListLight0, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
+  if ((st = launch_flatten(kListHeavy, parent, n, dst, (unsigned*)sa.tree_bits, d->sm_count, s))) return st;
+  if ((st = launch_scan(kHeavy, sa, d->sm_count, wl_slack, s))) return st;
   ra.phase = 1;
-  if ((st = enqueue_rounds(ra, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
+  if ((st = enqueue_rounds(ra, kListHeavy, m, d->sm_count, 0, d->round_grid, d->abl_grid, s, nullptr))) return st;
   return finish();
 }
 

@@ -72,7 +72,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
   const int thr = g.st->threshold;
   const bool vec = ((((uintptr_t)g.nlist) | ((uintptr_t)g.eweight)) & 15) == 0;
   const bool zero_vec = (((uintptr_t)g.inMST) & 3) == 0;
-  unsigned* ctr = &g.st->wl_count[KIND][0];
+  ListCount& list = g.st->lists[KIND == kLight ? kListLight0 : kListHeavy];
   if (threadIdx.x == 0) {
     sm.chunk = g.chunk;
     sm.kept = 0;
@@ -144,7 +144,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
     if (!total) continue;
     unsigned pos = 0, avail = 0, fresh = 0;
     if (lane == 0) {
-      chunk_take(&sm.chunk, g.chunk, ctr, total, pos, avail, fresh, g.st, g.wl_cap);
+      chunk_take(&sm.chunk, g.chunk, &list.slots, total, pos, avail, fresh, g.st, g.wl_cap);
       atomicAdd(&sm.kept, total);
     }
     pos = __shfl_sync(0xffffffffu, pos, 0);
@@ -166,7 +166,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
   const unsigned first = (unsigned)(sm.chunk >> 32);  // null entries in the slots not given out
   for (unsigned p = (unsigned)sm.chunk + threadIdx.x; p < g.chunk; p += kGroupThreads)
     if (first + p < g.wl_cap) g.wl0[first + p] = make_int4(-1, -1, 0, 0);
-  if (threadIdx.x == 0 && sm.kept) atomicAdd(&g.st->scan_kept[KIND], sm.kept);
+  if (threadIdx.x == 0 && sm.kept) atomicAdd(&list.kept, sm.kept);
 }
 
 // The rounds of one phase by the group, then the whole group again.
@@ -175,7 +175,8 @@ __device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, 
   BorArgs a{};
   a.phase = phase;
   a.nodes = g.nodes;
-  a.list = a.wl0 = g.wl0;
+  a.list = phase == 0 ? kListLight0 : kListHeavy;
+  a.wl0 = g.wl0;
   a.wl1 = g.wl1;
   a.wl_cap = g.wl_cap;
   a.parent = g.parent;
@@ -188,15 +189,19 @@ __device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, 
   a.min_tiles = g.min_tiles;
   a.count_atomics = g.count_atomics;
   BorState b = {};
-  b.W = min(ld_volatile(&g.st->wl_count[phase][0]), g.wl_cap);
+  b.W = min(ld_volatile(&g.st->lists[a.list].slots), g.wl_cap);
   b.first = 1;
   b.skip = skip;
   __syncthreads();  // the scan's use of the shared memory is over
   bor_smem_init(sm.bor);
   __syncthreads();
-  if (sy.rank == 0 && threadIdx.x == 0) g.st->t_round_start[phase] = globaltimer_ns();
+  if (sy.rank == 0 && threadIdx.x == 0) {
+    g.st->t_round_start[phase] = globaltimer_ns();
+    g.st->wl_count[phase][0] = b.W;
+    g.st->wl_kept[phase][0] = ld_volatile(&g.st->lists[a.list].kept);
+  }
   bool left;
-  bor_rounds<kGroupThreads, kGroupEpt, true>(a, b, true, sy, sm.bor, left);
+  bor_rounds<kGroupThreads, kGroupEpt, true, false>(a, b, sy, sm.bor, left);
   if (sy.rank == 0 && threadIdx.x == 0) g.st->rounds[phase] = b.r;
   return sy.regroup(left, (unsigned)phase + 1u);
 }

@@ -173,7 +173,7 @@ __host__ __device__ __forceinline__ float heuristic_log2_quantile(int n, int m) 
 // decoded quantile selects the light-phase threshold from the sorted weight
 // sample of the feature pass.
 __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sorted, int n, int m,
-                            ecl::DevState* st, float* feat_out) {
+                            ecl::DevState* st, float* feat_out, int lists) {
   // the whole parameter blob (21 KB) is staged in shared memory first, so the
   // layers read it at shared-memory latency instead of one global load per
   // multiply-add
@@ -221,6 +221,29 @@ __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sort
   } else {
     st->filtered = 0;
     st->threshold = 0x7fffffff;
+  }
+  // the lists' split weights, from the same sorted sample (read as unsigned:
+  // negative weights come after the others)
+  st->split_light = 0xffffffffu;
+  if (lists) {
+    auto count_le = [&](int w) {  // sample entries <= w, signed
+      int lo = 0, hi = kSample;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sorted[mid] <= w) lo = mid + 1;
+        else hi = mid;
+      }
+      return lo;
+    };
+    const int neg = count_le(-1), light = count_le(st->threshold);
+    float r0, r1;
+    ecl::split_ranks(n, m, st->filtered, (float)light / kSample, &r0, &r1);
+    auto ranked = [&](float r) { return (unsigned)sorted[((int)(r * kSample) + neg) % kSample]; };
+    if (r0 < 1.f) st->split_light = ranked(r0);
+    if (r1 < 1.f) {
+      st->split_heavy = ranked(r1);
+      st->mid = 1;
+    }
   }
   // output 1: log2 of the degree split, in [1, 6]
   st->learned_split = 1 << (int)lrintf(fminf(fmaxf(y[1], 1.f), 6.f));
@@ -390,8 +413,8 @@ int ecl_learned_sample(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t s) {
 
 // The features (sorted sample + k_prep's degree statistics) and the MLP, on
 // stream s once both are complete; writes the decoded schedule into the
-// solve's control block `st`.
-int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t s, void* st) {
+// solve's control block `st`, and where its lists are split if it has several.
+int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t s, void* st, int lists) {
   float *d_params, *d_feat;
   void* d_acc;
   int* d_sample;
@@ -400,7 +423,7 @@ int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t s, void* 
   int r = ecl_ctx_learned_buffers(c, &d_params, &d_feat, &d_acc, &d_sample, &version, &sms);
   if (r) return r;
   k_mlp_apply<<<1, 256, 0, s>>>(d_params, (const FeatAcc*)d_acc, d_sample, g->nodes, g->edges,
-                               (ecl::DevState*)st, d_feat);
+                               (ecl::DevState*)st, d_feat, lists);
   ML_TRY(cudaGetLastError());
   return ECL_OK;
 }

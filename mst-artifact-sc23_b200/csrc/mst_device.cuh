@@ -8,22 +8,17 @@
 // built in a light phase (w <= threshold, signed compare as at :172) and a
 // heavy phase (w > threshold). Launch sequence of one solve:
 //
-//   k_prep        initPM + CSR checks + threshold choice + the tile->vertex
-//                 table of the edge-balanced scans
-//   k_scan<L,E>   initWL<true>: a producer warp stages CSR tiles into shared
-//                 memory with bulk asynchronous copies; every consumer lane
-//                 takes E consecutive entries, so rows shorter than E stay
-//                 inside one lane and longer rows are spread over lanes,
-//                 warps and CTAs (the reference's thread/warp degree split,
-//                 :167/:185, becomes the entries-per-lane E). Also zeroes
-//                 inMST. Appends are warp-aggregated, reserved in chunks.
+//   k_prep        initPM + CSR checks + threshold choice + the task->row table
+//                 of the scans
+//   k_scan, light  initWL<true> (scan_device.cuh). Also zeroes inMST
 //   k_round       the phase's Boruvka rounds in one cooperative launch
 //                 (rounds_device.cuh: kernel1, kernel2, kernel3 per round,
 //                 bounded grid barriers, no host round trip per round), and
 //   k_round_tail  its last rounds on one thread-block cluster. The ablation
 //                 switches run the variants in k_rounds instead.
-//   k_flatten     parent[v] = root(v) once after the light phase
-//   k_scan<H,E>   initWL<false>: keeps heavy entries across light trees
+//   k_flatten     parent[v] = root(v) once after the light phase, and a bit per
+//                 vertex of its largest tree
+//   k_scan, heavy  initWL<false>: keeps heavy entries across light trees
 //   k_round, k_round_tail   heavy phase
 #pragma once
 #include <cuda_pipeline.h>
@@ -38,7 +33,7 @@
 namespace ecl {
 
 constexpr int kThreads = 512;          // threads of the prep and flatten kernels
-constexpr int kGran = 128;             // entries per tile->vertex table step (the smallest scan warp range)
+constexpr int kGran = 512;             // entries of a scan task, and per step of the task->row table
 // Round CTAs of 1024 threads, two per SM (measured on RMAT-22: 2.4 % faster
 // with the learned schedule and 4.6 % with the heuristic one than 512 x 4;
 // 256 x 8 was 11-15 % slower)
@@ -74,29 +69,7 @@ constexpr int kSplitAfter = 8;         // find steps before path splitting start
 #ifndef ECL_FLAT_ROUNDS
 #define ECL_FLAT_ROUNDS 2
 #endif
-#ifndef ECL_L2_HINTS
-#define ECL_L2_HINTS 1                 // evict-first CSR streams, evict-last parent gathers in the scans
-#endif
-// Entries per lane of the heavy scan: 0 takes the light scan's (the split's),
-// 4, 8 or 16 fixes it. Its parent[] gathers make the heavy scan latency-bound,
-// and E = 4 runs the most consumer warps per SM (4 CTAs of 8): measured on
-// RMAT-25 11.6 % faster than the split's E = 8 (RMAT-22 4.6 %), no slower on
-// ER, grid or RGG graphs.
-#ifndef ECL_HEAVY_EPT
-#define ECL_HEAVY_EPT 4
-#endif
 constexpr unsigned long long kBarrierTimeoutNs = 5ull * 1000 * 1000 * 1000;
-
-// Entries per thread of the edge-balanced scan for a degree split: rows
-// shorter than the split stay inside one thread.
-__host__ __device__ __forceinline__ int scan_ept(int split) {
-  return split <= 4 ? 4 : (split <= 8 ? 8 : 16);
-}
-
-// Entries per lane of the heavy scan (ECL_HEAVY_EPT, else the split's).
-__host__ __device__ __forceinline__ int heavy_ept(int split) {
-  return ECL_HEAVY_EPT ? ECL_HEAVY_EPT : scan_ept(split);
-}
 
 struct PrepArgs {
   int nodes, edges;
@@ -105,10 +78,12 @@ struct PrepArgs {
   int* parent;
   u64* minv0;
   u64* minv1;
-  int* first_v;  // [tiles + 1]: vertex holding entry t * kGran; last = nodes - 1
+  int* first_v;  // [tiles + 1]: row holding entry t * kGran; last = nodes - 1
   int tiles;     // ceil(edges / kGran)
   int mode, explicit_thr, split;
   float quantile;
+  int use_lists;   // the light and heavy entries may be split into several lists
+  int both_slots;  // minv1 is a min array too (the ablation variants)
   DevState* st;
   FeatAcc* feat;  // learned schedule: degree statistics gathered here, else null
 };
@@ -121,14 +96,13 @@ struct ScanArgs {
   const int* first_v;
   int tiles;
   int* parent;
-  int4* wl;
+  const unsigned* tree_bits;  // bit v: v lies in the light phase's largest tree
+  int4* wl0;
+  int4* wl1;
   unsigned wl_cap;
   unsigned char* inMST;
-  int vec_ok;    // nlist / eweight 16-byte aligned
   int zero_vec;  // inMST 16-byte aligned
-  int sm_count;  // host side: sizes the persistent scan launch
-  unsigned wl_slack;  // host side: wl_cap minus the most entries a scan can keep
-  unsigned chunk;     // worklist slots a warp reserves at once (set at launch)
+  unsigned chunk;     // worklist slots a CTA reserves at once (set at launch)
   int ids;            // 1 = append CSR indices (int) instead of tuples (kAblNoTuples)
   DevState* st;
 };
@@ -259,523 +233,123 @@ __device__ void choose_threshold(const PrepArgs& a, int* samp) {
   }
 }
 
+// The lists' split weights from k_prep's own sample of kThreads weights (one CTA): the sample
+// of a wanted rank is the one with that many below it.
+__device__ void choose_lists(const PrepArgs& a, int* samp) {
+  DevState* st = a.st;
+  const int tid = threadIdx.x;
+  __syncthreads();
+  const int thr = st->threshold, filtered = st->filtered;
+  const uint64_t h = ecl_mix64(0xC1A55000ull + (uint64_t)tid);
+  const int w = a.eweight[(unsigned)(h % (uint64_t)(unsigned)a.edges)];
+  samp[tid] = w;
+  const int light = __syncthreads_count(w <= thr);
+  float r0, r1;
+  split_ranks(a.nodes, a.edges, filtered, (float)light / kThreads, &r0, &r1);
+  int below = 0;
+  for (int i = 0; i < kThreads; i++) below += (unsigned)samp[i] < (unsigned)w || (samp[i] == w && i < tid);
+  if (below == (int)(r0 * kThreads)) st->split_light = (unsigned)w;
+  if (below == (int)(r1 * kThreads)) {
+    st->split_heavy = (unsigned)w;
+    st->mid = 1;
+  }
+  if (tid == 0 && r0 >= 1.f) st->split_light = 0xffffffffu;
+}
+
 __global__ void __launch_bounds__(kThreads) k_prep(PrepArgs a) {
   __shared__ int samp[4096];
   DevState* st = a.st;
-  if (blockIdx.x == 0) choose_threshold(a, samp);
+  if (blockIdx.x == 0) {
+    choose_threshold(a, samp);
+    if (a.mode != ECL_THRESH_LEARNED) {
+      if (a.use_lists) choose_lists(a, samp);
+      else if (threadIdx.x == 0) st->split_light = 0xffffffffu;
+    }
+  }
   const int n = a.nodes, m = a.edges;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   bool bad = false;
   FeatPart fp;  // degree statistics (learned schedule)
-  for (int v = gid; v < n; v += stride) {
-    a.parent[v] = v;
-    a.minv0[v] = kNoEdge;
-    a.minv1[v] = kNoEdge;
-    const int b = __ldg(a.nindex + v), e = __ldg(a.nindex + v + 1);
-    const bool row_bad = b < 0 || e < b || e > m;
-    bad |= row_bad;
-    if (a.feat) fp.add(e > b ? (unsigned)(e - b) : 0u);
-    // Tile->vertex table (first_v[t] = row of entry t * kGran), first step:
-    // the row holding the first step position at or after its start writes
-    // itself there (each position has exactly one owner, so no conflicts);
-    // the positions further inside long rows stay 0 and are filled by a max
-    // scan (k_fill_chunks, k_fill_carry), rows being in increasing order.
-    const unsigned t0 = ((unsigned)b + kGran - 1) / kGran, t1 = ((unsigned)e + kGran - 1) / kGran;
-    if (!row_bad && t0 < t1) a.first_v[t0] = v;
+  const int lane = threadIdx.x & 31;
+  for (long long first = gid - lane; first < n; first += stride) {
+    const int base = (int)first;
+    const int v = first + lane < n ? base + lane : n;
+    unsigned t0 = 0, t1 = 0;  // the table steps that start inside row v
+    if (v < n) {
+      a.parent[v] = v;
+      a.minv0[v] = kNoEdge;
+      if (a.both_slots) a.minv1[v] = kNoEdge;
+      const int b = __ldg(a.nindex + v), e = __ldg(a.nindex + v + 1);
+      const bool row_bad = b < 0 || e < b || e > m;
+      bad |= row_bad;
+      if (a.feat) fp.add(e > b ? (unsigned)(e - b) : 0u);
+      if (!row_bad) {
+        t0 = ((unsigned)b + kGran - 1) / kGran;
+        t1 = ((unsigned)e + kGran - 1) / kGran;
+      }
+    }
+    // Task->row table: every row writes itself at the steps it holds, a long
+    // row with the whole warp.
+    if (t1 - t0 <= 4)
+      for (unsigned t = t0; t < t1; t++) a.first_v[t] = v;
+    for (unsigned longs = __ballot_sync(0xffffffffu, t1 - t0 > 4); longs; longs &= longs - 1) {
+      const int src = __ffs(longs) - 1;
+      const unsigned f = __shfl_sync(0xffffffffu, t0, src), l = __shfl_sync(0xffffffffu, t1, src);
+      for (unsigned t = f + lane; t < l; t += 32) a.first_v[t] = base + src;
+    }
   }
-  if (gid == 0) bad |= __ldg(a.nindex) != 0 || __ldg(a.nindex + n) != m;
+  if (gid == 0) {
+    a.first_v[a.tiles] = n - 1;
+    bad |= __ldg(a.nindex) != 0 || __ldg(a.nindex + n) != m;
+  }
   if (bad) atomicOr(&st->error, kErrFormat);
   if (a.feat) fp.fold<kThreads>(a.feat);  // uniform across the grid
 }
 
-// Inclusive max scan of the tile->vertex table first_v[0 .. tiles), in
-// chunks of kFillChunk entries: each CTA scans its chunk and records the
-// chunk's maximum; k_fill_carry then raises every chunk to the maximum of the
-// chunks before it and writes the end sentinel first_v[tiles] = nodes - 1.
-constexpr int kFillChunk = 8192;  // 1024 threads x 8 entries
-
-__global__ void __launch_bounds__(1024) k_fill_chunks(int* t, int count, int* chunk_max) {
-  __shared__ int warp_max[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long base = (long long)blockIdx.x * kFillChunk + threadIdx.x * 8;
-  int x[8], run = 0;
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    x[q] = base + q < count ? t[base + q] : 0;
-    run = max(run, x[q]);
-    x[q] = run;
-  }
-  int incl = run;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl = max(incl, y);
-  }
-  if (lane == 31) warp_max[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    int w = warp_max[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w = max(w, y);
-    }
-    warp_max[lane] = w;
-  }
-  __syncthreads();
-  int before = __shfl_up_sync(0xffffffffu, incl, 1);
-  if (lane == 0) before = 0;
-  if (warp > 0) before = max(before, warp_max[warp - 1]);
-#pragma unroll
-  for (int q = 0; q < 8; q++)
-    if (base + q < count) t[base + q] = max(x[q], before);
-  if (threadIdx.x == 0) chunk_max[blockIdx.x] = warp_max[31];
-}
-
-__global__ void __launch_bounds__(1024) k_fill_carry(int* t, int count, const int* chunk_max, int nodes) {
-  __shared__ int carry;
-  if (threadIdx.x < 32) {
-    int c = 0;
-    for (int i = threadIdx.x; i < (int)blockIdx.x; i += 32) c = max(c, chunk_max[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
-    if (threadIdx.x == 0) carry = c;
-  }
-  __syncthreads();
-  const long long base = (long long)blockIdx.x * kFillChunk;
-  if (carry > 0)
-    for (int q = threadIdx.x; q < kFillChunk && base + q < count; q += blockDim.x)
-      t[base + q] = max(t[base + q], carry);
-  if (blockIdx.x == 0 && threadIdx.x == 0) t[count] = nodes - 1;
-}
-
-// ------------------------------------------------------------------ scans
 enum ScanKind { kLight = 0, kHeavy = 1 };
 
-// Edge-balanced CSR scan (initWL, ECL_MST.cu:157-207), warp-specialised and
-// persistent. A tile is kScanWarps * 32 * EPT consecutive CSR entries. One
-// producer warp stages each tile's slices of nlist, eweight and nindex into a
-// ring of shared-memory stages with bulk asynchronous copies (cp.async.bulk;
-// completion counted on the stage's `full` mbarrier) and refills a stage once
-// every consumer warp has released it (`empty` mbarrier). Each consumer warp
-// takes 32 * EPT consecutive entries of the staged tile, EPT per lane, so hub
-// rows and short rows cost the same per entry (the reference's thread / warp
-// degree split, :167/:185, becomes the entries-per-lane EPT). A consumer
-// finds the vertex of its entries from the staged nindex slice alone: a
-// 32-ary search for the row holding the warp's first entry, the rows starting
-// inside the warp's range marked in a warp-private array, and a warp max-scan
-// over the marks; no step waits on the whole CTA. One-direction entries
-// (nlist[j] > v) passing the phase's weight test are appended as
-// {rep(v), rep(n), w, j}; the heavy scan also drops entries whose endpoints
-// share a light-phase tree (parent[] is flat, so a rep is one load).
-// Worklist slots are reserved per warp, `chunk` at a time, from the phase's
-// counter; the unused tail of each warp's last chunk is filled with null
-// entries (x = -1), which the first round skips.
-constexpr int kScanWarps = 8;                        // consumer warps of a scan CTA
-constexpr int kScanThreads = (kScanWarps + 1) * 32;  // plus the producer warp
-#ifndef ECL_SCAN_SEGCAP
-#define ECL_SCAN_SEGCAP 2048
-#endif
-constexpr int kScanSegCap = ECL_SCAN_SEGCAP;         // longest nindex slice (vertices) staged per tile
-constexpr unsigned kScanMaxChunk = 64;               // worklist slots a warp reserves at once
-
-// ring stages and the resident CTAs per SM the launch bounds ask for, per EPT
-#ifndef ECL_SCAN_S4
-#define ECL_SCAN_S4 2
-#endif
-#ifndef ECL_SCAN_S8
-#define ECL_SCAN_S8 2
-#endif
-#ifndef ECL_SCAN_S16
-#define ECL_SCAN_S16 2
-#endif
-#ifndef ECL_SCAN_B4
-#define ECL_SCAN_B4 4
-#endif
-#ifndef ECL_SCAN_B8
-#define ECL_SCAN_B8 3
-#endif
-#ifndef ECL_SCAN_B16
-#define ECL_SCAN_B16 2
-#endif
-constexpr int kScanStages[3] = {ECL_SCAN_S4, ECL_SCAN_S8, ECL_SCAN_S16};
-constexpr int kScanMinB[3] = {ECL_SCAN_B4, ECL_SCAN_B8, ECL_SCAN_B16};
-
-template <int EPT>
-struct ScanCfg {
-  static constexpr int kIdx = EPT == 4 ? 0 : (EPT == 8 ? 1 : 2);
-  static constexpr int kTile = kScanWarps * 32 * EPT;  // entries per tile
-  static constexpr int kStages = kScanStages[kIdx];
-  static constexpr int kMinBlocks = kScanMinB[kIdx];
-  static constexpr int kSegInts = kScanSegCap + 8;         // slice from a 16-byte boundary
-  static constexpr int kStageInts = 2 * kTile + kSegInts;  // nlist, eweight, nindex slice
-  static constexpr size_t kHead = 128 + 48 * kStages;      // mbarriers, then stage headers
-  // stages, then one row-mark array of 32 * EPT ints per consumer warp
-  static constexpr size_t kSmem = kHead + sizeof(int) * ((size_t)kStages * kStageInts + kTile);
-};
-
-template <int EPT>
-constexpr size_t scan_smem_bytes() {
-  return ScanCfg<EPT>::kSmem;
-}
-
-struct ScanStage {
-  int v_lo;  // vertex holding the tile's first entry
-  int span;  // vertices v_lo .. v_lo + span - 1 may own the tile's entries
-  int off;   // nindex[v_lo] is at slice index off
-  int seg;   // 1 = nindex[v_lo .. v_lo + span] is staged
-  int wfirst[kScanWarps];  // vertex holding each consumer warp's first entry
-};
-static_assert(sizeof(ScanStage) == 48, "stage header size");
-
-// Largest v in [lo, lo + span) with nindex[v] <= e, for an entry e of a tile
-// whose rows are v_lo .. v_lo + span - 1 (global binary search; used when the
-// tile's slice is too long to stage).
-__device__ __forceinline__ int vertex_in(const int* nindex, int lo, int span, long long e) {
-  int hi = lo + span;
-  while (hi - lo > 1) {
-    const int mid = lo + ((hi - lo) >> 1);
-    if ((long long)__ldg(nindex + mid) <= e) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// The tiles a scan CTA takes, in order: first, first + step, ... < end.
-struct TileSeq {
-  int first, step, end;
-};
-__device__ __forceinline__ TileSeq scan_tiles(int ntiles) {
-#ifdef ECL_SCAN_CONTIG
-  const int g = gridDim.x, b = blockIdx.x, per = ntiles / g, rem = ntiles % g;
-  const int first = b * per + min(b, rem);
-  return TileSeq{first, 1, first + per + (b < rem ? 1 : 0)};
-#else
-  return TileSeq{(int)blockIdx.x, (int)gridDim.x, ntiles};
-#endif
-}
-
-// Producer warp: fills stage i % kStages with the CTA's i-th tile. The
-// 16-byte aligned bulk of each slice goes by bulk copy; a ragged end (the
-// last tile, the end of nindex) or unaligned arrays go by plain copies of the
-// warp's lanes, published by the same mbarrier arrival.
-template <int EPT>
-__device__ void scan_produce(const ScanArgs& a, unsigned char* smem, int ntiles) {
-  using C = ScanCfg<EPT>;
-  u64* full = reinterpret_cast<u64*>(smem);
-  u64* empty = full + C::kStages;
-  ScanStage* hdr = reinterpret_cast<ScanStage*>(smem + 128);
-  int* stages = reinterpret_cast<int*>(smem + C::kHead);
-  const int lane = threadIdx.x & 31;
-  const int n = a.nodes, m = a.edges;
-  const bool edge_bulk = a.vec_ok != 0;
-  const bool idx_bulk = (((uintptr_t)a.nindex) & 15) == 0;
-  const u64 stream_pol = l2_policy_evict_first();  // the CSR is read once per scan
-  // Lanes 0..7 read the vertex of each consumer warp's first entry, lane 8
-  // the vertex of the next tile's first entry (first_v has one entry per
-  // kGran entries), one tile ahead of the copies.
-  const TileSeq ts = scan_tiles(ntiles);
-  auto first_of = [&](int t) -> int {
-    if (lane > kScanWarps || t >= ts.end) return 0;
-    const int tb = t * (C::kTile / kGran) + lane * (32 * EPT / kGran);
-    return __ldg(a.first_v + min(tb, a.tiles));
-  };
-  int i = 0;
-  int cur = first_of(ts.first);
-  for (int t = ts.first; t < ts.end; t += ts.step, i++) {
-    const int s = i % C::kStages;
-    const int nxt = first_of(t + ts.step);
-    // every lane waits; the warp goes on only if all lanes saw the phase end
-    if (i >= C::kStages &&
-        !__all_sync(0xffffffffu, mbar_wait(&empty[s], ((i / C::kStages) - 1) & 1, kBarrierTimeoutNs))) {
-      if (lane == 0) atomicOr(&a.st->error, kErrTimeout);
-      break;
+// parent[v] = root(v) for every vertex, before a list of unmapped vertices and
+// before the heavy scan, and a bit per vertex of the largest tree so far (a
+// word per warp and 32 vertices). Four walks per thread run in lock step,
+// their loads in flight together; they read through L1, where the few vertices
+// near a giant tree's root stay (a value from before another thread's store is
+// a lower ancestor of the same root, so a stale line only lengthens a walk).
+__global__ void __launch_bounds__(kThreads) k_flatten(int* parent, int n, const DevState* st, unsigned* tree_bits,
+                                                      int list) {
+  constexpr int U = 4;
+  if (list == kListHeavy ? !st->filtered : !st->lists[list].slots) return;  // nothing follows that reads it
+  if (ld_volatile(&st->error) & (kErrFormat | kErrTimeout)) return;
+  const int giant = st->giant, lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (kThreads / 32), w0 = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  for (long long base = (long long)w0 * (32 * U); base < n; base += (long long)warps * (32 * U)) {
+    int v[U], first[U], p[U];
+    bool walk[U];
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      v[i] = (int)base + i * 32 + lane;
+      walk[i] = base + i * 32 + lane < n;
+      first[i] = p[i] = walk[i] ? __ldcg(parent + v[i]) : -1;
+      walk[i] = walk[i] && p[i] != v[i];
     }
-    const int v_lo = __shfl_sync(0xffffffffu, cur, 0);
-    const int v_hi = __shfl_sync(0xffffffffu, cur, kScanWarps);
-    if (lane < kScanWarps) hdr[s].wfirst[lane] = cur;
-    cur = nxt;
-    const int span = v_hi - v_lo + 1;
-    const bool seg = span <= kScanSegCap;
-    const long long j0 = (long long)t * C::kTile;
-    const int cnt = (int)min((long long)C::kTile, (long long)m - j0);
-    int* nl = stages + (size_t)s * C::kStageInts;
-    int* ew = nl + C::kTile;
-    int* sx = ew + C::kTile;
-    const int a0 = v_lo & ~3, off = v_lo - a0;
-    const int want = seg ? off + span + 1 : 0;  // slice ints from a0 (a0 + want <= n + 1)
-    const int bulk_e = edge_bulk ? (cnt & ~3) : 0;
-    const int bulk_x = idx_bulk ? min((want + 3) & ~3, (n + 1 - a0) & ~3) : 0;
-    for (int q = bulk_e + lane; q < cnt; q += 32) {
-      nl[q] = __ldg(a.nlist + j0 + q);
-      ew[q] = __ldg(a.eweight + j0 + q);
-    }
-    for (int q = bulk_x + lane; q < want; q += 32) sx[q] = __ldg(a.nindex + a0 + q);
-    if (lane == 0) {
-      hdr[s].v_lo = v_lo;
-      hdr[s].span = span;
-      hdr[s].off = off;
-      hdr[s].seg = seg ? 1 : 0;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_tx(&full[s], 4u * (unsigned)(2 * bulk_e + bulk_x));
-      if (bulk_e) {
-        if (ECL_L2_HINTS) {
-          bulk_g2s_hint(nl, a.nlist + j0, 4u * (unsigned)bulk_e, &full[s], stream_pol);
-          bulk_g2s_hint(ew, a.eweight + j0, 4u * (unsigned)bulk_e, &full[s], stream_pol);
-        } else {
-          bulk_g2s(nl, a.nlist + j0, 4u * (unsigned)bulk_e, &full[s]);
-          bulk_g2s(ew, a.eweight + j0, 4u * (unsigned)bulk_e, &full[s]);
+    for (bool any = true; any;) {
+      any = false;
+      int gp[U];
+#pragma unroll
+      for (int i = 0; i < U; i++) gp[i] = walk[i] ? ld_ca(parent + p[i]) : 0;
+#pragma unroll
+      for (int i = 0; i < U; i++)
+        if (walk[i]) {
+          if (gp[i] == p[i]) walk[i] = false;
+          else any = true;
+          p[i] = gp[i];
         }
-      }
-      if (bulk_x) bulk_g2s(sx, a.nindex + a0, 4u * (unsigned)bulk_x, &full[s]);
-    }
-  }
-  // Copies still in flight land before the CTA may exit.
-  if (lane == 0)
-    for (int k = max(0, i - C::kStages); k < i; k++)
-      if (!mbar_wait(&full[k % C::kStages], (k / C::kStages) & 1, kBarrierTimeoutNs))
-        atomicOr(&a.st->error, kErrTimeout);
-}
-
-// One parent[] gather of the heavy scan, through L2 with the evict-last
-// policy (L1-allocating loads measured no faster: the gathers rarely repeat
-// within an SM).
-__device__ __forceinline__ int gather_parent(const int* p, u64 policy) {
-  return ECL_L2_HINTS ? ld_cg_hint(p, policy) : __ldg(p);
-}
-
-template <int KIND, int EPT>
-__global__ void __launch_bounds__(kScanThreads, ScanCfg<EPT>::kMinBlocks) k_scan(ScanArgs a) {
-  using C = ScanCfg<EPT>;
-  constexpr int kTile = C::kTile, R = 32 * EPT;  // entries per tile / per consumer warp
-  extern __shared__ __align__(128) unsigned char scan_dyn[];
-  u64* full = reinterpret_cast<u64*>(scan_dyn);
-  u64* empty = full + C::kStages;
-  const ScanStage* hdr = reinterpret_cast<const ScanStage*>(scan_dyn + 128);
-  const int* stages = reinterpret_cast<const int*>(scan_dyn + C::kHead);
-  DevState* st = a.st;
-  if (ld_volatile(&st->error) & kErrFormat) return;  // set by k_prep only
-  if (KIND == kHeavy && !st->filtered) return;
-  // only the variant the split selects runs
-  if ((KIND == kHeavy ? heavy_ept(st->split) : scan_ept(st->split)) != EPT) return;
-  const int n = a.nodes, m = a.edges;
-  const int ntiles = (int)(((long long)m + kTile - 1) / kTile);
-  if ((int)blockIdx.x >= ntiles) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kStages; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kScanWarps);
-    }
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (warp == kScanWarps) {
-    scan_produce<EPT>(a, scan_dyn, ntiles);
-    return;
-  }
-  // Row-start marks of this warp's range: row index minus the warp's first
-  // row, 0 = no row starts there. Each lane clears its own slots after use.
-  int* rmark = reinterpret_cast<int*>(scan_dyn + C::kHead) + (size_t)C::kStages * C::kStageInts + warp * R;
-  for (int q = lane; q < R; q += 32) rmark[q] = 0;
-  __syncwarp();
-  const int thr = st->threshold;
-  const u64 keep_pol = l2_policy_evict_last();  // parent[] is gathered by every consumer warp
-  unsigned* ctr = &st->wl_count[KIND][0];
-  unsigned wpos = 0, wend = 0, kept = 0;  // this warp's reserved, unused slots [wpos, wend)
-  unsigned idmax = 0;                     // largest neighbour id seen, as unsigned
-  int i = 0;
-  const TileSeq ts = scan_tiles(ntiles);
-  for (int t = ts.first; t < ts.end; t += ts.step, i++) {
-    const int s = i % C::kStages;
-    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (i / C::kStages) & 1, kBarrierTimeoutNs))) {
-      if (lane == 0) atomicOr(&st->error, kErrTimeout);
-      break;
-    }
-    const int* nl = stages + (size_t)s * C::kStageInts;
-    const int v_lo = hdr[s].v_lo, span = hdr[s].span;
-    const int* sx = nl + 2 * kTile + hdr[s].off;  // sx[i] = nindex[v_lo + i]
-    // entry positions fit in 32 bits (edges < 2^31)
-    const unsigned jw = (unsigned)t * kTile + warp * R;  // first entry of this warp
-    const unsigned jl = jw + lane * EPT;                 // first entry of this lane
-    const int lim = jl < (unsigned)m ? min(EPT, m - (int)jl) : 0;  // the lane's valid entries
-    const int* nlw = nl + warp * R + lane * EPT;
-    const int* eww = nlw + kTile;
-    // the lane's entries, 128 bits at a time from the staged tile
-    int nb[EPT], w[EPT];
-    if (lim == EPT) {
-#pragma unroll
-      for (int q = 0; q < EPT; q += 4) {
-        const int4 x = *reinterpret_cast<const int4*>(nlw + q);
-        const int4 y = *reinterpret_cast<const int4*>(eww + q);
-        nb[q] = x.x; nb[q + 1] = x.y; nb[q + 2] = x.z; nb[q + 3] = x.w;
-        w[q] = y.x; w[q + 1] = y.y; w[q + 2] = y.z; w[q + 3] = y.w;
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < EPT; q++) {
-        nb[q] = q < lim ? nlw[q] : -1;
-        w[q] = q < lim ? eww[q] : 0;
-      }
-    }
-    // Vertex of every entry, as an offset from v_lo.
-    int vi[EPT];
-    if (hdr[s].seg) {
-      const int lo = hdr[s].wfirst[warp] - v_lo;  // row holding entry jw
-      // Rows starting inside (jw, jw + R) mark their start; of several rows
-      // starting at one position (zero-degree rows) the last one owns it.
-      if (jw < (unsigned)m)
-        for (int kb = lo + 1;; kb += 32) {
-          const int k = kb + lane;
-          const unsigned sk = k <= span ? (unsigned)sx[k] : jw + R;
-          const bool in = sk < jw + R;
-          if (in) atomicMax(&rmark[sk - jw], k - lo);
-          if (__ballot_sync(0xffffffffu, in) != 0xffffffffu) break;
-        }
-      __syncwarp();
-      // an entry's row is the last mark at or before it (lane-local running
-      // maximum, then a warp exclusive max-scan across lanes)
-      int run = 0, loc[EPT];
-#pragma unroll
-      for (int q = 0; q < EPT; q += 4) {
-        int4* slot = reinterpret_cast<int4*>(&rmark[lane * EPT + q]);
-        const int4 mk = *slot;
-        *slot = make_int4(0, 0, 0, 0);
-        loc[q] = run = max(run, mk.x);
-        loc[q + 1] = run = max(run, mk.y);
-        loc[q + 2] = run = max(run, mk.z);
-        loc[q + 3] = run = max(run, mk.w);
-      }
-      int incl = run;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl = max(incl, x);
-      }
-      int prev = __shfl_up_sync(0xffffffffu, incl, 1);
-      if (lane == 0) prev = 0;
-#pragma unroll
-      for (int q = 0; q < EPT; q++) vi[q] = lo + max(prev, loc[q]);
-    } else {
-      // slice too long to stage (long runs of zero-degree vertices)
-#pragma unroll
-      for (int q = 0; q < EPT; q++) vi[q] = q < lim ? vertex_in(a.nindex, v_lo, span, jl + q) - v_lo : 0;
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);  // this warp reads nothing more of the stage
-    if (KIND == kLight && lim > 0) {  // inMST = 0 (the reference memsets it, :306)
-      if (a.zero_vec && lim == EPT) {
-        if (EPT == 4) *reinterpret_cast<unsigned*>(a.inMST + jl) = 0u;
-        else if (EPT == 8) *reinterpret_cast<uint2*>(a.inMST + jl) = make_uint2(0u, 0u);
-        else *reinterpret_cast<uint4*>(a.inMST + jl) = make_uint4(0u, 0u, 0u, 0u);
-      } else {
-        for (int q = 0; q < lim; q++) a.inMST[jl + q] = 0;
-      }
-    }
-    // filter: one direction with a valid id (v < nb < n, as one unsigned
-    // compare), then the phase's weight test
-    unsigned cand = 0;
-    int vtx[EPT], nrep[EPT];
-#pragma unroll
-    for (int q = 0; q < EPT; q++) {
-      const int v = v_lo + vi[q];
-      if (q < lim) idmax = max(idmax, (unsigned)nb[q]);
-      const bool pass = q < lim && (unsigned)nb[q] - (unsigned)v - 1u < (unsigned)(n - v - 1) &&
-                        (KIND == kLight ? w[q] <= thr : w[q] > thr);
-      cand |= (unsigned)pass << q;
-      vtx[q] = v;
-      nrep[q] = nb[q];
-    }
-    if (KIND == kHeavy) {  // light-tree reps of both endpoints, all loads in flight together
-      // A lane's entries run in CSR order, so consecutive ones mostly share
-      // their row: its rep is loaded once per row, not once per entry.
-      int rv = -1, rrep = 0;
-#pragma unroll
-      for (int q = 0; q < EPT; q++)
-        if (cand & (1u << q)) {
-          if (vtx[q] != rv) {
-            rv = vtx[q];
-            rrep = gather_parent(a.parent + rv, keep_pol);
-          }
-          vtx[q] = rrep;
-          nrep[q] = gather_parent(a.parent + nb[q], keep_pol);
-        }
-#pragma unroll
-      for (int q = 0; q < EPT; q++)
-        if (vtx[q] == nrep[q]) cand &= ~(1u << q);
-    }
-    const unsigned cnt = __popc(cand);
-    // warp reservation: slots from this warp's chunk, then a fresh chunk
-    unsigned incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += x;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total) {
-      const unsigned avail = wend - wpos;
-      unsigned fresh = 0, take = 0;
-      if (total > avail) {
-        take = max(total - avail, a.chunk);
-        if (lane == 0) fresh = atomicAdd(ctr, take);
-        fresh = __shfl_sync(0xffffffffu, fresh, 0);
-      }
-      unsigned p = incl - cnt;
-#pragma unroll
-      for (int q = 0; q < EPT; q++) {
-        if (!(cand & (1u << q))) continue;
-        const unsigned slot = p < avail ? wpos + p : fresh + (p - avail);
-        if (slot >= a.wl_cap) atomicOr(&st->error, kErrOverflow);
-        else if (a.ids) reinterpret_cast<int*>(a.wl)[slot] = (int)(jl + q);
-        else a.wl[slot] = make_int4(vtx[q], nrep[q], w[q], (int)(jl + q));
-        p++;
-      }
-      if (total > avail) {
-        wpos = fresh + (total - avail);
-        wend = fresh + take;
-      } else {
-        wpos += total;
-      }
-      kept += cnt;
-    }
-  }
-  if (idmax >= (unsigned)n) atomicOr(&st->error, kErrFormat);  // a neighbour id outside [0, n)
-  for (unsigned p = wpos + lane; p < wend; p += 32)  // null entries in the unused slots
-    if (p < a.wl_cap) {
-      if (a.ids) reinterpret_cast<int*>(a.wl)[p] = -1;
-      else a.wl[p] = make_int4(-1, -1, 0, 0);
     }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
-  if (lane == 0 && kept) atomicAdd(&st->scan_kept[KIND], kept);
-}
-
-// parent[v] = root(v) for every vertex, once before the heavy scan.
-// A per-CTA set of roots already found ends a walk as soon as it reaches one:
-// every walk through a giant light tree would otherwise read that tree's
-// root entry, one L2 line hammered by millions of threads. Roots do not
-// change during the pass (other threads only shorten paths).
-__global__ void __launch_bounds__(kThreads) k_flatten(int* parent, int n, const DevState* st) {
-  constexpr int kRootSlots = 1024;
-  __shared__ int roots[kRootSlots];
-  if (!st->filtered || (ld_volatile(&st->error) & (kErrFormat | kErrTimeout))) return;
-  for (int i = threadIdx.x; i < kRootSlots; i += blockDim.x) roots[i] = -1;
-  __syncthreads();
-  volatile int* known = roots;
-  auto slot = [](int x) { return ((unsigned)x * 0x85EBCA6Bu) >> 22; };  // 10 bits
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    int x = v, p = __ldcg(parent + v);
-    while (p != x) {
-      x = p;
-      if (known[slot(x)] == x) break;
-      p = __ldcg(parent + x);
+    for (int i = 0; i < U; i++) {
+      if (p[i] >= 0 && p[i] != first[i]) __stcg(parent + v[i], p[i]);
+      const unsigned word = __ballot_sync(0xffffffffu, p[i] == giant);
+      if (lane == 0 && base + i * 32 < n) tree_bits[(base >> 5) + i] = word;
     }
-    known[slot(x)] = x;
-    if (x != v) __stcg(parent + v, x);
   }
 }
 
@@ -785,7 +359,7 @@ __global__ void __launch_bounds__(kThreads) k_flatten(int* parent, int n, const 
 // every entry's parent read, min-slot guard read, atomicMin and reset on one
 // L2 address; these small direct-mapped tables absorb the repeats per CTA.
 struct RoundSmem {
-  ReserveSmem rs;            // the CTA's warp totals
+  unsigned warp_off[32][2];  // the CTA's warp totals
   unsigned cursor;           // entries this CTA kept so far in the current find/min pass
   int seg_n;                 // segments of the list the passes read (1 = dense from seg_off[0])
   unsigned seg_q[kMaxRoundCtas + 1];  // entries in the segments before b (seg_q[seg_n] = all)
@@ -863,10 +437,10 @@ __device__ __forceinline__ void seg_load(RoundSmem& s, const DevState* st, int n
     const unsigned x = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += x;
   }
-  if (lane == 31) s.rs.warp_off[warp][0] = incl;
+  if (lane == 31) s.warp_off[warp][0] = incl;
   __syncthreads();
   unsigned q = incl - mine;
-  for (int w = 0; w < warp; w++) q += s.rs.warp_off[w][0];
+  for (int w = 0; w < warp; w++) q += s.warp_off[w][0];
 #pragma unroll
   for (int k = 0; k < kSegPer; k++) {
     const int b = b0 + k;
@@ -1363,11 +937,17 @@ __global__ void __launch_bounds__(kRoundThreads, ECL_ROUND_MIN_BLOCKS) k_rounds(
   // endpoints are gathered as they are).
   const bool fresh0 = !(a.abl & kAblNoTuples);
   const bool ndd = (a.abl & kAblNoDD) != 0;
-  if (stamp) st->t_round_start[ph] = globaltimer_ns();
+  const ListCount list = st->lists[ph == 0 ? kListLight0 : kListHeavy];
+  const unsigned first = min(list.slots, a.wl_cap);
+  if (stamp) {
+    st->t_round_start[ph] = globaltimer_ns();
+    st->wl_count[ph][0] = first;
+    st->wl_kept[ph][0] = list.kept;
+  }
   for (;;) {
-    unsigned W = min(ld_volatile(&st->wl_count[ph][r]), a.wl_cap);
+    unsigned W = r == 0 ? first : min(ld_volatile(&st->wl_count[ph][r]), a.wl_cap);
     if (W == 0) break;  // (kAblNoDD: no entry joined two trees last round)
-    if (ndd) W = min(ld_volatile(&st->wl_count[ph][0]), a.wl_cap);  // the phase's whole list, every round
+    if (ndd) W = first;  // the phase's whole list, every round
     if (r >= ECL_MAX_ROUNDS) {
       if (stamp) atomicOr(&st->error, kErrRounds);
       break;
@@ -1418,7 +998,7 @@ __global__ void __launch_bounds__(kRoundThreads, ECL_ROUND_MIN_BLOCKS) k_rounds(
                    fresh, start, stride, s, flat);
     if (fresh && blockIdx.x == 0 && threadIdx.x == 0) {  // the scan's list is round 0's output
       st->wl_count[ph][1] = W;
-      st->wl_kept[ph][1] = st->scan_kept[ph];
+      st->wl_kept[ph][1] = list.kept;
     }
     if (!fresh && !tail && !ndd && threadIdx.x == 0) {  // this CTA's segment of the output list
       st->seg_cnt[blockIdx.x] = s.cursor;
@@ -1450,15 +1030,19 @@ __global__ void __launch_bounds__(kRoundThreads, ECL_ROUND_MIN_BLOCKS) k_rounds(
 // ------------------------------------------------ reference ablation steps
 // kAblNoTuples: the vertex of every CSR entry (the reference's NoTuples
 // variant keeps such an slist, Deoptimizations/..._NoTuples.cu:163-169),
-// filled entry-parallel from the scans' tile->vertex table (the row holding
-// entry t * kGran), then a short walk along nindex.
+// filled entry-parallel: a binary search in nindex between the rows the
+// scans' task->row table gives.
 __global__ void __launch_bounds__(kThreads) k_slist(const int* nindex, const int* first_v, int* slist,
                                                     int edges, const DevState* st) {
   if (ld_volatile(&st->error) & kErrFormat) return;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < edges; j += gridDim.x * blockDim.x) {
-    int v = __ldg(first_v + j / kGran);
-    while (__ldg(nindex + v + 1) <= j) v++;
-    slist[j] = v;
+    int lo = __ldg(first_v + j / kGran), hi = __ldg(first_v + j / kGran + 1);
+    while (lo < hi) {  // the last row starting at or before j
+      const int mid = lo + ((hi - lo + 1) >> 1);
+      if (__ldg(nindex + mid) <= j) lo = mid;
+      else hi = mid - 1;
+    }
+    slist[j] = lo;
   }
 }
 

@@ -1,7 +1,6 @@
 // Device building blocks of the B200 ECL-MST engine: coherent loads, the
-// bounded grid barrier, CTA-aggregated worklist reservation, find with path
-// halving and the CAS union. Shared by the single-graph engine (ecl_mst.cu)
-// and the batched engine.
+// bounded grid barrier, bulk copies, find with path halving and the CAS union.
+// Shared by the single-graph engine (ecl_mst.cu) and the batched engine.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -26,8 +25,6 @@ enum : unsigned {
 // writes its kept entries as one segment of the round's output list.
 constexpr int kMaxRoundCtas = 1024;
 
-constexpr int kChunkLog = 7;  // long rows are scanned in aligned 128-entry chunks
-constexpr int kChunk = 1 << kChunkLog;
 constexpr u64 kNoEdge = ~0ull;
 
 // Degree statistics of the learned schedule's features, summed over all
@@ -103,6 +100,20 @@ struct BorState {
   int skip;    // the tree that offers nothing, -1 = none
 };
 
+// The worklists a solve's scans build, in the order their rounds run. The light
+// phase's entries may be split by weight into two lists, and the light scan may
+// set aside the lightest of the heavy phase's: rounds on a short list of the
+// lightest entries first leave most of the later ones inside one tree. Each
+// list holds the smaller weights of its phase as unsigned, so the forest is the
+// phase's. Lists 1 and 2 grow down from the end of the two arrays, beside the
+// space the rounds before them compact into:
+//   wl0:  [light 0, then heavy ...      ... light 1]
+//   wl1:  [                             ...     mid]
+enum : int { kListLight0 = 0, kListLight1 = 1, kListMid = 2, kListHeavy = 3 };
+struct ListCount {
+  unsigned slots, kept;  // slots reserved (null padding included), entries
+};
+
 // Control block of one solve, zeroed before every solve.
 struct DevState {
   int threshold;       // light phase keeps w <= threshold
@@ -112,8 +123,6 @@ struct DevState {
   unsigned bar_count;  // grid barrier: CTAs arrived in the current generation
   unsigned bar_gen;    // grid barrier: generation counter
   int rounds[2];       // Boruvka rounds per phase
-  unsigned desc_count; // long-row chunk descriptors emitted by the current scan
-  unsigned pad;
   float quantile;      // learned / quantile modes: filter quantile in [0,1]
   int learned_split;   // learned mode: predicted degree split
   u64 atomics;         // guarded atomicMin issued (stats mode)
@@ -122,21 +131,48 @@ struct DevState {
   // [phase][2r] after round r's find/min pass, [phase][2r+1] after its mark pass
   u64 t_round_start[2];
   u64 t_round[2][2 * ECL_MAX_ROUNDS];
-  unsigned scan_kept[2];  // entries each scan kept (wl_count[p][0] also counts padding)
-  unsigned wl_kept[2][ECL_MAX_ROUNDS + 1];  // [phase][r + 1] = entries round r kept (no padding)
+  ListCount lists[4];
+  unsigned split_light;  // light entries up to this weight (as unsigned) go to list light 0
+  unsigned split_heavy;  // heavy entries up to this weight go to list mid, if
+  int mid;               // that list is used
+  int lists_bad;         // the lists of one array overlap (more entries than it holds)
+  unsigned wl_kept[2][ECL_MAX_ROUNDS + 1];  // [phase][r] = entries entering round r (no padding)
   // The last find/min pass's output list, one segment per CTA: CTA b wrote
   // seg_cnt[b] entries from position seg_off[b] (written before the grid
   // barrier that ends the pass, read after it).
   unsigned seg_cnt[kMaxRoundCtas];
   unsigned seg_off[kMaxRoundCtas];
-  unsigned root_cnt[2][3];  // [phase][pass % 3] = live roots a roots pass kept
+  unsigned root_cnt[4][3];  // [list][pass % 3] = live roots a roots pass kept
   BorState resume;          // where the cluster kernel goes on with the phase
-  unsigned bar[2];          // GridSync counters: k_round's by phase; k_group's
+  unsigned bar[4];          // GridSync counters: k_round's by list; k_group's
   unsigned gate;            // the last gate opened (GridSync::regroup)
   unsigned gate_target;
   unsigned graph;           // batch: the graph the cluster works on
   int giant;                // the light phase's largest tree (by a vote of sampled vertices)
 };
+
+// Weights at which a solve's lists are split (kListLight0 ...), as the shares
+// of the graph's entries at or below them (2 = no split).
+//   Light entries: the first kSplitLight x n go to list light 0, the others to
+// light 1, if these are half as many at least and all of them kSplitMin. The
+// rounds on half an entry per vertex leave few trees for the others, which then
+// drop out at their first look; but the short list's last rounds cost their
+// latency, 100-150 us (ER 3M, 4.4M light entries: 0.99 ms against 1.06, 1.21 at
+// 0.25 x n; RMAT-18 unfiltered, 3.8M: 0.38 against 0.50; ER 1.2M, 1.7M: 0.66
+// against 0.57).
+//   Heavy entries: list mid takes them up to kSplitHeavy x n entries in all,
+// where the slots and parents of the vertices outgrow L2, so that every entry
+// the heavy scan keeps costs DRAM accesses (ER 16M 7.7 ms against 8.9, RMAT-25
+// 10.8 against 11.7; RMAT-22, in L2, 1.55 against 1.52).
+constexpr float kSplitLight = 0.5f, kSplitHeavy = 2.0f;
+constexpr int kSplitMin = 3 << 20;
+constexpr int kMidNodes = 1 << 23;
+__device__ __forceinline__ void split_ranks(int n, int m, int filtered, float light_share, float* rank0, float* rank1) {
+  const float half = 0.5f * (float)m;
+  const float f0 = kSplitLight * (float)n / half, f1 = kSplitHeavy * (float)n / half;
+  *rank0 = f0 * 1.5f < light_share && light_share * half >= (float)kSplitMin ? f0 : 2.f;
+  *rank1 = filtered && n >= kMidNodes && f1 > 1.3f * light_share && f1 <= 0.4f ? f1 : 2.f;
+}
 
 __device__ __forceinline__ u64 globaltimer_ns() {
   u64 t;
@@ -182,6 +218,14 @@ __device__ __forceinline__ bool grid_barrier(DevState* st, u64 timeout_ns, unsig
   return (ld_volatile(&st->error) & kErrTimeout) == 0;
 }
 
+// 32-bit global load through L1, for data that no CTA writes between two
+// barriers (or where an older value will do).
+__device__ __forceinline__ int ld_ca(const int* p) {
+  int v;
+  asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // ---- mbarriers and bulk asynchronous copies (cp.async.bulk, no multicast)
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -194,10 +238,6 @@ __device__ __forceinline__ void mbar_init(u64* bar, unsigned count) {
 // Makes barrier initialisation visible to the asynchronous copy unit.
 __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(u64* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 // Arrive and add `bytes` to the transaction count the phase waits for.
@@ -236,20 +276,9 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Global -> shared bulk copy of `bytes` (multiple of 16, both addresses
-// 16-byte aligned); completion is counted on `bar`.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, u64* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
-
 // ---- L2 eviction priorities (createpolicy + .L2::cache_hint, sm_80 and
-// later). Streams read once (the CSR in the scans) are marked evict-first so
-// they do not push out the small arrays every thread gathers from (parent[],
-// the min slots), which are marked evict-last where they are read.
+// later): the CSR, read once per scan, is marked evict-first, the small array
+// every warp of the heavy scan gathers from (parent[]) evict-last.
 __device__ __forceinline__ u64 l2_policy_evict_first() {
   u64 p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -262,7 +291,8 @@ __device__ __forceinline__ u64 l2_policy_evict_last() {
   return p;
 }
 
-// Global -> shared bulk copy as bulk_g2s, with an L2 cache policy.
+// Global -> shared bulk copy of `bytes` (a multiple of 16, both addresses
+// 16-byte aligned) with an L2 cache policy; completion is counted on `bar`.
 __device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, unsigned bytes, u64* bar, u64 policy) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
@@ -276,72 +306,6 @@ __device__ __forceinline__ int ld_cg_hint(const int* p, u64 policy) {
   int v;
   asm volatile("ld.global.cg.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
   return v;
-}
-
-// 32-bit global load through L1, for data that no CTA writes between two
-// barriers (or where an older value will do).
-__device__ __forceinline__ int ld_ca(const int* p) {
-  int v;
-  asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Shared memory of one CTA-wide two-counter reservation.
-struct ReserveSmem {
-  unsigned warp_off[32][2];
-  unsigned base[2];
-};
-
-// CTA-aggregated reservation of c0 slots in counter ctr0 and c1 slots in
-// counter ctr1 (ctr1 may be null when every c1 is 0): one warp-shuffle scan,
-// one scan over warp totals and at most one global atomic per counter per CTA.
-// Every thread of the CTA must call it (it contains __syncthreads).
-__device__ __forceinline__ void cta_reserve2(unsigned c0, unsigned c1, unsigned* ctr0,
-                                             unsigned* ctr1, ReserveSmem& sm, unsigned& pos0,
-                                             unsigned& pos1) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned s0 = c0, s1 = c1;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned t0 = __shfl_up_sync(0xffffffffu, s0, o);
-    const unsigned t1 = __shfl_up_sync(0xffffffffu, s1, o);
-    if (lane >= o) {
-      s0 += t0;
-      s1 += t1;
-    }
-  }
-  if (lane == 31) {
-    sm.warp_off[warp][0] = s0;
-    sm.warp_off[warp][1] = s1;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    const unsigned w0 = lane < nw ? sm.warp_off[lane][0] : 0u;
-    const unsigned w1 = lane < nw ? sm.warp_off[lane][1] : 0u;
-    unsigned x0 = w0, x1 = w1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned t0 = __shfl_up_sync(0xffffffffu, x0, o);
-      const unsigned t1 = __shfl_up_sync(0xffffffffu, x1, o);
-      if (lane >= o) {
-        x0 += t0;
-        x1 += t1;
-      }
-    }
-    if (lane < nw) {
-      sm.warp_off[lane][0] = x0 - w0;
-      sm.warp_off[lane][1] = x1 - w1;
-    }
-    if (lane == 31) {
-      sm.base[0] = x0 ? atomicAdd(ctr0, x0) : 0u;
-      sm.base[1] = x1 ? atomicAdd(ctr1, x1) : 0u;
-    }
-  }
-  __syncthreads();
-  pos0 = sm.base[0] + sm.warp_off[warp][0] + (s0 - c0);
-  pos1 = sm.base[1] + sm.warp_off[warp][1] + (s1 - c1);
-  __syncthreads();
 }
 
 // Union-find order. A root is hooked under a root of higher priority, where

@@ -38,9 +38,9 @@ constexpr unsigned kTailEntries = 32768;
 
 struct BorArgs {
   int phase, nodes;
-  const int4* list;        // the phase's entries, dense
-  int4* wl0;               // compacted lists, in turn: wl1, wl0, wl1, ...
-  int4* wl1;               // (`list` may be wl0 itself)
+  int list;                // kList*: the entries the rounds start from
+  int4* wl0;
+  int4* wl1;
   unsigned wl_cap;
   int* parent;
   u64* minv;               // all kNoEdge between phases
@@ -399,25 +399,32 @@ __device__ __forceinline__ void bor_roots_step(const BorArgs& a, const int (&v)[
 }
 
 // Rounds from state `b` until the list is empty (true) or, grid-wide, until
-// it is at most a.tail entries long (false: `b` is where to go on). `fresh`:
-// the first list's endpoints are roots and differ. CTAs beyond what a round
-// needs leave (`left`); their `b` is meaningless.
+// it is at most a.tail entries long (false: `b` is where to go on). The
+// endpoints of the lists light 0 and heavy are roots that differ: their first
+// round finds nothing and compacts nothing (without kLists there are no others).
+// CTAs beyond what a round needs leave (`left`); their `b` is meaningless.
 //
 // Below some 10^5 entries a round is bound by its dependent L2 accesses (0.35
 // us a load or atomic) and barriers, so the loads that do not depend on each
 // other are issued together, the entries of a CTA with one tile stay in
 // registers from the offer to the mark pass (kKeep: not in k_round, whose 32
-// registers a thread they would spill, 2 % slower on RMAT-22), and where the vertices are few
-// for the threads at work the roots pass looks at all of them instead of
-// keeping a list.
-template <int T, int E, bool kKeep, class Sync>
-__device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool fresh_list, Sync& sy, BorSmem& s,
-                                           bool& left) {
+// registers a thread they would spill, 2 % slower on RMAT-22), and where the
+// vertices are few for the threads at work the roots pass looks at all of them
+// instead of keeping a list.
+template <int T, int E, bool kKeep, bool kLists, class Sync>
+__device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, Sync& sy, BorSmem& s, bool& left) {
   constexpr int N = 2 * E;
   constexpr unsigned tile = T * E;
   DevState* st = a.st;
   const int ph = a.phase, tid = threadIdx.x;
   left = false;
+  // The list, and the arrays the rounds compact into in turn: never the one
+  // whose end still holds the list, or a later one that fits beside it.
+  const bool fresh_list = !kLists || a.list == kListLight0 || a.list == kListHeavy;
+  const bool mid = kLists && a.list == kListMid;
+  int4* const out0 = mid ? a.wl0 : a.wl1;
+  int4* const out1 = mid ? a.wl1 : a.wl0;
+  const int4* first_list = fresh_list ? a.wl0 : out1 + (a.wl_cap - st->lists[a.list].slots);
   unsigned atomics = 0;
   const bool stamp = sy.rank == 0 && tid == 0;
   bool done = true;
@@ -449,8 +456,8 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     }
     const unsigned start = sy.rank, stride = sy.active;
     const bool fresh = b.first && fresh_list;
-    const int4* in = b.k == 0 ? a.list : ((b.k & 1) ? a.wl1 : a.wl0);
-    int4* out = (b.k & 1) ? a.wl0 : a.wl1;
+    const int4* in = b.k == 0 ? first_list : ((b.k & 1) ? out0 : out1);
+    int4* out = (b.k & 1) ? out1 : out0;
     const unsigned W = b.W, ntiles = (W + tile - 1) / tile;
     const unsigned region = share_region(W, tile, start, stride);
     const bool one = kKeep && ntiles <= stride;  // no CTA has a second tile
@@ -519,7 +526,7 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
     }
     if (stamp && fresh) {  // the scan's list is the first round's output
       st->wl_count[ph][b.r + 1] = W;
-      st->wl_kept[ph][b.r + 1] = st->scan_kept[ph];
+      st->wl_kept[ph][b.r + 1] = ld_volatile(&st->lists[a.list].kept);
     }
     for (int i = tid; i < kHotSlots; i += T) {  // flush the partial minima
       const int r = s.hot_rep[i];
@@ -592,7 +599,7 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
                                                        : wanted(W2, stride) * T;
     int* rout = scan_roots(ahead) ? nullptr : ((b.flips & 1) ? a.roots1 : a.roots0);
     const int* rin = (b.flips & 1) ? a.roots0 : a.roots1;
-    unsigned* rctr = &st->root_cnt[ph][b.flips % 3];
+    unsigned* rctr = &st->root_cnt[a.list][b.flips % 3];
     int flip = 0;
     constexpr int U = E > 1 ? 4 : 2;
     if (b.first && !all) {  // few entries for the vertices: take the roots from this CTA's entries
@@ -626,7 +633,7 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, bool f
         bor_roots_step<U>(a, v, valid, false, b.skip, rout, rctr, flip, s);
       }
     }
-    if (stamp) st->root_cnt[ph][(b.flips + 1) % 3] = 0;  // the next roots pass's counter
+    if (stamp) st->root_cnt[a.list][(b.flips + 1) % 3] = 0;  // the next roots pass's counter
     if (tid == 0) s.cursor = 0;
     if (!sy.sync()) break;
     if (stamp) st->t_round[ph][2 * b.r - 1] = globaltimer_ns();
@@ -651,18 +658,36 @@ __global__ void __launch_bounds__(kBorThreads, kBorBlocks) k_round(BorArgs a) {
   DevState* st = a.st;
   if (a.phase == 1 && !st->filtered) return;
   if (ld_volatile(&st->error) & (kErrFormat | kErrTimeout)) return;  // bits no CTA of this kernel sets before a barrier
+  // every CTA finds the same: the lists of one array must not meet
+  const unsigned l0 = st->lists[kListLight0].slots, l1 = st->lists[kListLight1].slots, l2 = st->lists[kListMid].slots;
+  const bool first = a.list == kListLight0;
+  if (first ? (u64)l0 + l1 > a.wl_cap || (u64)max(l0, l1) + l2 > a.wl_cap : st->lists_bad != 0) {
+    if (first && blockIdx.x == 0 && threadIdx.x == 0) {
+      atomicOr(&st->error, kErrOverflow);
+      st->lists_bad = 1;
+      st->resume = BorState{};
+    }
+    return;
+  }
   BorState b = {};
-  b.W = min(ld_volatile(&st->wl_count[a.phase][0]), a.wl_cap);
+  b.W = min(st->lists[a.list].slots, a.wl_cap);
+  b.r = st->rounds[a.phase];
   b.first = 1;
-  b.skip = a.phase == 1 ? st->giant : -1;
+  b.skip = first ? -1 : st->giant;
   GridSync sy;
-  sy.init(st, &st->bar[a.phase]);
+  sy.init(st, &st->bar[a.list]);
   bor_smem_init(s);
   __syncthreads();
   const bool stamp = sy.rank == 0 && threadIdx.x == 0;
-  if (stamp) st->t_round_start[a.phase] = globaltimer_ns();
+  if (stamp) {
+    if (b.r == 0) st->t_round_start[a.phase] = globaltimer_ns();
+    if (b.W && b.r < ECL_MAX_ROUNDS) {
+      st->wl_count[a.phase][b.r] = b.W;
+      st->wl_kept[a.phase][b.r] = st->lists[a.list].kept;
+    }
+  }
   bool left;
-  const bool done = bor_rounds<kBorThreads, kBorEpt, false>(a, b, true, sy, s, left);
+  const bool done = bor_rounds<kBorThreads, kBorEpt, false, true>(a, b, sy, s, left);
   if (stamp && !left) {
     st->rounds[a.phase] = b.r;
     if (done) b.W = 0;
@@ -670,10 +695,9 @@ __global__ void __launch_bounds__(kBorThreads, kBorBlocks) k_round(BorArgs a) {
   }
 }
 
-// The end of a phase on one cluster: goes on from where k_round stopped. After
-// the light phase its first CTA also names the tree that holds most of the
-// vertices (a vote of sampled vertices), which the heavy phase's rounds then
-// leave out of their offers.
+// The end of a list on one cluster: goes on from where k_round stopped. Its
+// first CTA then names the tree that holds most of the vertices (a vote of
+// sampled vertices), which the next list's rounds leave out of their offers.
 __global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads, 1) k_round_tail(BorArgs a) {
   __shared__ BorSmem s;
   DevState* st = a.st;
@@ -690,10 +714,12 @@ __global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads
       bor_seg_load<kTailThreads>(s, st, b.nseg);
       __syncthreads();
     }
-    bor_rounds<kTailThreads, kTailEpt, true>(a, b, true, sy, s, left);
+    bor_rounds<kTailThreads, kTailEpt, true, true>(a, b, sy, s, left);
     if (sy.rank == 0 && threadIdx.x == 0 && !left) st->rounds[a.phase] = b.r;
   }
-  if (a.phase == 0 && st->filtered && sy.rank == 0) {
+  const bool more = a.list == kListLight0 ? st->filtered || st->lists[kListLight1].slots
+                                          : a.list != kListHeavy && st->lists[a.list].slots;
+  if (more && sy.rank == 0) {
     __syncthreads();
     int* vote = reinterpret_cast<int*>(s.seg_q);
     const int v = (int)(uf_prio((int)threadIdx.x + 1) % (unsigned)a.nodes);
