@@ -427,11 +427,6 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster(ClArgs g) {
 }
 
 // ------------------------------------------------------------------ batch
-struct GraphDesc {
-  long long nindex_off, edge_off;
-  int nodes, edges;
-};
-
 // One size class of a batch: `count` graphs, largest first, each solved by
 // the next free cluster. Every cluster has its own control block and its own
 // share of the scratch pools, for graphs of up to `cap` vertices and entries.

@@ -27,6 +27,10 @@ int ecl_learned_sample(ecl_mst_ctx* c, const ecl_graph* d_graph, cudaStream_t s)
 int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* d_graph, cudaStream_t s, void* st, int lists);
 int ecl_learned_upload(ecl_mst_ctx* c, cudaStream_t s);
 unsigned ecl_learned_weights_version();
+// The same for the graphs of a batch, all in two launches.
+int ecl_learned_batch_prepare();
+int ecl_learned_batch(ecl_mst_ctx* c, const ecl::GraphDesc* graphs, int count, int least, const int* nindex,
+                      const int* eweight, ecl::FeatAcc* acc, ecl::LearnedChoice* choice, cudaStream_t s);
 
 using namespace ecl;
 
@@ -1448,6 +1452,20 @@ __global__ void k_or_error(const DevState* src, DevState* dst) {
 
 constexpr int kBatchDefaultCap = 1 << 19;
 constexpr int kMaxLargeStreams = 8;      // concurrent streams for a batch's large graphs
+// Graphs of up to kTeamEdges entries are solved by teams (k_batch_group) where
+// at least kTeamMin of a batch's large graphs are that small, or half as many
+// and no others; the rest by the engines, K streams side by side. 39 large
+// graphs (17 by teams) 8.45 -> 7.95 ms on 8 streams, 33 (18) 6.36 -> 5.59, 55
+// (53) 5.57 -> 3.62, 5 (5) 1.07 -> 0.97. Two graphs alone are the faster on the
+// engines (0.22 ms against 0.27), and three by teams before five others only
+// delay those (2.05 -> 2.15). With kTeamEdges 2^22 the largest graph of a team
+// takes as long as on the whole chip alone (8.44 ms, 5.65, 3.54). Teams of fewer
+// than kTeamMinCtas CTAs gain nothing, and on one stream a graph has the chip
+// to itself as it is.
+constexpr int kTeamEdges = 1 << 21;
+constexpr int kTeamMin = 8;
+constexpr int kTeamMinCtas = 6;
+constexpr int64_t kTeamGraphCost = 1 << 18;  // of the rounds' latency, in entries
 constexpr int kDefaultLargeStreams = 4;  // measured: 957 large graphs of the mixed batch 1.5x faster than on one
 
 }  // namespace
@@ -1479,6 +1497,14 @@ struct ecl_batch_ctx {
   // more streams (opts batch_large_streams)
   ecl_mst_ctx* big[kMaxLargeStreams] = {};
   cudaEvent_t large_fork = nullptr, large_join[kMaxLargeStreams] = {};
+  // the graphs that teams of CTAs solve (k_batch_group): descriptors, degree
+  // statistics and learned schedules by graph, barriers and control blocks by team
+  GraphDesc* d_team_graphs = nullptr;
+  FeatAcc* d_team_feat = nullptr;
+  LearnedChoice* d_team_choice = nullptr;
+  TeamWords* d_team_words = nullptr;
+  DevState* d_team_states = nullptr;
+  int team_grid = 0;
   cudaEvent_t ev[3] = {};
   // the large-graph launch sequence captured as a CUDA graph, keyed by the batch
   cudaGraphExec_t exec = nullptr;
@@ -1515,6 +1541,11 @@ extern "C" void ecl_batch_ctx_destroy(ecl_batch_ctx* c) {
   cudaFree(c->states);
   cudaFree(c->d_graphs);
   cudaFree(c->d_queue);
+  cudaFree(c->d_team_graphs);
+  cudaFree(c->d_team_feat);
+  cudaFree(c->d_team_choice);
+  cudaFree(c->d_team_words);
+  cudaFree(c->d_team_states);
   cudaFree(c->st);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
@@ -1570,8 +1601,17 @@ extern "C" int ecl_batch_ctx_create(int device, int32_t max_graphs, int64_t max_
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->large_fork, cudaEventDisableTiming)))) return fail(st);
   for (auto& e : c->large_join)
     if ((st = cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)))) return fail(st);
-  if (max_graph_edges > c->cap || max_graph_nodes > c->cap)
+  if (max_graph_edges > c->cap || max_graph_nodes > c->cap) {
     if ((st = batch_big_ctx(c, 0))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&c->d_team_graphs, (size_t)max_graphs * sizeof(GraphDesc))))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&c->d_team_feat, (size_t)max_graphs * sizeof(FeatAcc))))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&c->d_team_choice, (size_t)max_graphs * sizeof(LearnedChoice))))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&c->d_team_words, kMaxTeams * sizeof(TeamWords))))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&c->d_team_states, kMaxTeams * sizeof(DevState))))) return fail(st);
+    if ((st = ecl_learned_batch_prepare())) return fail(st);
+    c->team_grid = coop_grid((const void*)k_batch_group, kGroupThreads, c->sm_count);
+    if (c->team_grid <= 0) return fail(ECL_ERR_CUDA);
+  }
   *out = c;
   return ECL_OK;
 }
@@ -1662,6 +1702,116 @@ int batch_small(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& sm
   return ECL_OK;
 }
 
+// Which graphs a batch's teams solve, on what scratch and how many CTAs.
+struct TeamPlan {
+  std::vector<GraphDesc> descs;  // by team
+  Team team[kMaxTeams + 1];
+  int teams = 0, ctas = 0;
+};
+
+// `graphs` (largest first) on as many teams as the scratch of `engines` engines
+// has room for: every graph goes to the team with the least work so far, a
+// team's share of the CTAs is its share of the work, and a graph's work is its
+// entries and kTeamGraphCost for the rounds' latency.
+TeamPlan plan_teams(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& graphs, int engines, int max_ctas) {
+  TeamPlan plan;
+  const int total_ctas = c->team_grid;
+  int T = (int)std::min<size_t>(graphs.size(), (size_t)std::min(kMaxTeams, total_ctas / kTeamMinCtas));
+  auto cap_of = [&](int g) { return b->edges[g] + std::min<int64_t>(b->edges[g], kWlSlack) / 4; };
+  for (;; T--) {  // (one team always fits)
+    // no more teams than lists fit: team t's first graph, its largest, is graph t
+    int64_t room = 0;
+    for (int t = 0; t < T; t++) room += cap_of(graphs[t]);
+    if (T > 1 && room > engines * (int64_t)c->big[0]->wl_cap) continue;
+    std::vector<std::vector<int>> lists(T);
+    std::vector<int64_t> work(T, 0);
+    std::vector<int> nmax(T, 0);
+    for (int g : graphs) {
+      const int t = (int)(std::min_element(work.begin(), work.end()) - work.begin());
+      lists[t].push_back(g);
+      work[t] += b->edges[g] + kTeamGraphCost;
+      nmax[t] = std::max(nmax[t], b->nodes[g]);
+    }
+    // the teams' scratch, first fit
+    std::vector<int64_t> slots_used(engines, 0), wl_used(engines, 0);
+    bool fits = true;
+    for (int t = 0; t < T && fits; t++) {
+      const int64_t n = nmax[t], cap = cap_of(lists[t][0]);
+      int k = 0;
+      while (k < engines && (slots_used[k] + n > c->max_nodes || wl_used[k] + cap > c->big[k]->wl_cap)) k++;
+      if (!(fits = k < engines)) break;
+      Team& tm = plan.team[t];  // 20 bytes of slots a vertex, from an 8-byte boundary
+      tm.slots = reinterpret_cast<u64*>(static_cast<char*>(c->big[k]->slots) + 20 * slots_used[k]);
+      tm.wl0 = c->big[k]->wl[0] + wl_used[k];
+      tm.wl1 = c->big[k]->wl[1] + wl_used[k];
+      tm.wl_cap = (unsigned)cap;
+      slots_used[k] += (n + 1) & ~1;
+      wl_used[k] += cap;
+    }
+    if (!fits) continue;
+    int64_t total = 0;
+    for (int64_t w : work) total += w;
+    std::vector<int> ctas(T);
+    int used = 0;
+    for (int t = 0; t < T; t++) {
+      ctas[t] = std::max(1, std::min(max_ctas, (int)((total_ctas - T) * work[t] / total)));
+      used += ctas[t];
+    }
+    for (; used < total_ctas; used++) {  // the rest one by one to the team with the most work per CTA
+      int best = -1;
+      for (int t = 0; t < T; t++)
+        if (ctas[t] < max_ctas && (best < 0 || work[t] * ctas[best] > work[best] * ctas[t])) best = t;
+      if (best < 0) break;
+      ctas[best]++;
+    }
+    for (int t = 0; t < T; t++) {
+      plan.team[t].first_graph = (int)plan.descs.size();
+      plan.team[t].first_cta = plan.ctas;
+      plan.ctas += ctas[t];
+      for (int g : lists[t]) plan.descs.push_back(GraphDesc{b->nindex_off[g], b->edge_off[g], b->nodes[g], b->edges[g]});
+    }
+    plan.team[T] = Team{};
+    plan.team[T].first_graph = (int)plan.descs.size();
+    plan.team[T].first_cta = plan.ctas;
+    plan.teams = T;
+    return plan;
+  }
+}
+
+// The plan's graphs, whose descriptors are in c->d_team_graphs.
+int batch_teams(ecl_batch_ctx* c, const ecl_batch* b, const TeamPlan& plan, bool learned, uint8_t* d_inMST,
+                const mst_opts* o, cudaStream_t s) {
+  TeamArgs ta{};
+  ta.graphs = c->d_team_graphs;
+  ta.choice = c->d_team_choice;
+  ta.teams = plan.teams;
+  for (int t = 0; t <= plan.teams; t++) ta.team[t] = plan.team[t];
+  ta.learned_min = kLearnedMinEdges;
+  ta.words = c->d_team_words;
+  ta.states = c->d_team_states;
+  ta.nindex = b->nindex;
+  ta.nlist = b->nlist;
+  ta.eweight = b->eweight;
+  ta.inMST = d_inMST;
+  ta.st = c->st;
+  ta.mode = o->threshold_mode;
+  ta.explicit_thr = o->threshold;
+  ta.split = o->degree_split > 0 ? o->degree_split : kDefaultSplit;
+  ta.quantile = o->quantile;
+  ta.solo = o->small_tail < 0 ? 0u : (o->small_tail == 0 ? kDefaultSmallTail : (unsigned)o->small_tail);
+  if (o->flags & ECL_FLAG_NO_SMALL_TAIL) ta.solo = 0;
+  ta.min_tiles = o->round_min_tiles < 0 ? 0 : (o->round_min_tiles == 0 ? kDefaultMinTiles : o->round_min_tiles);
+  ta.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
+  ECL_CUDA_TRY(cudaMemsetAsync(c->d_team_words, 0, kMaxTeams * sizeof(TeamWords), s));
+  ECL_CUDA_TRY(cudaMemsetAsync(c->d_team_states, 0, kMaxTeams * sizeof(DevState), s));
+  if (learned) {
+    const int r = ecl_learned_batch(c->big[0], c->d_team_graphs, (int)plan.descs.size(), kLearnedMinEdges, b->nindex,
+                                    b->eweight, c->d_team_feat, c->d_team_choice, s);
+    if (r) return r;
+  }
+  return launch_ex(k_batch_group, plan.ctas, kGroupThreads, 0, s, true, nullptr, ta);
+}
+
 int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const mst_opts* o,
                   cudaStream_t s, bool timed, ecl_batch_stats* stats) {
   const int G = b->num_graphs;
@@ -1687,9 +1837,9 @@ int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const 
   if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   bool replayed = false;
   if (!large.empty()) {
-    // The large graphs' launch sequence (per graph: control-block reset and
-    // six kernels, no host round trip) is captured once per batch layout as a
-    // CUDA graph and replayed; if capture is unavailable it is enqueued.
+    // The large graphs' launch sequence (no host round trip) is captured once
+    // per batch layout as a CUDA graph and replayed; if capture is unavailable
+    // it is enqueued.
     std::vector<long long> key;
     key.push_back((long long)(uintptr_t)b->nindex);
     key.push_back((long long)(uintptr_t)b->nlist);
@@ -1738,8 +1888,15 @@ int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const 
     }
     if (K > 1 && lo.ctas_per_sm == 0) lo.ctas_per_sm = 1;
     key.push_back(K);  // the streams in use (fewer than asked when memory ran short)
-    std::vector<int> order(large);
+    std::vector<int> order(large), team;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->edges[x] > b->edges[y]; });
+    if (K > 1 && !round_ablation(lo.flags)) {
+      const auto rest = std::find_if(order.begin(), order.end(), [&](int g) { return b->edges[g] <= kTeamEdges; });
+      if (order.end() - rest >= (rest == order.begin() ? kTeamMin / 2 : kTeamMin)) {
+        team.assign(rest, order.end());
+        order.erase(rest, order.end());
+      }
+    }
     std::vector<int> lane_of(order.size());
     {
       std::vector<int64_t> load(K, 0);
@@ -1749,7 +1906,18 @@ int batch_enqueue(ecl_batch_ctx* c, const ecl_batch* b, uint8_t* d_inMST, const 
         load[k] += b->edges[order[i]];
       }
     }
+    TeamPlan plan;
+    if (!team.empty() && !(c->exec && c->exec_key == key)) {
+      plan = plan_teams(c, b, team, K, lo.ctas_per_sm > 0 ? lo.ctas_per_sm * c->sm_count : INT_MAX);
+      ECL_CUDA_TRY(cudaMemcpyAsync(c->d_team_graphs, plan.descs.data(), plan.descs.size() * sizeof(GraphDesc),
+                                   cudaMemcpyHostToDevice, s));
+    }
     auto enqueue_large = [&](cudaStream_t q) -> int {
+      if (!team.empty()) {
+        const int r = batch_teams(c, b, plan, learned, d_inMST, &lo, q);
+        if (r) return r;
+      }
+      if (order.empty()) return ECL_OK;
       if (K > 1) {
         ECL_CUDA_TRY(cudaEventRecord(c->large_fork, q));
         for (int k = 0; k < K; k++) ECL_CUDA_TRY(cudaStreamWaitEvent(c->big[k]->stream, c->large_fork, 0));

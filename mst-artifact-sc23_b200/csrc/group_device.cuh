@@ -203,7 +203,7 @@ __device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, 
   bool left;
   bor_rounds<kGroupThreads, kGroupEpt, true, false>(a, b, sy, sm.bor, left);
   if (sy.rank == 0 && threadIdx.x == 0) g.st->rounds[phase] = b.r;
-  return sy.regroup(left, (unsigned)phase + 1u);
+  return sy.regroup(left);
 }
 
 // One solve; the control block's counters are zero. False if a barrier timed
@@ -267,8 +267,109 @@ __device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) k_group(GroupArgs g) {
   __shared__ GroupSmem sm;
   GridSync sy;
-  sy.init(g.st, &g.st->bar[0]);
+  sy.init(g.st, g.st->bar, blockIdx.x, gridDim.x);
   group_solve(g, sy, sm);
+}
+
+// ------------------------------------------------------------------ batch
+// A batch's mid-size graphs (too large for a cluster) by teams of CTAs side by
+// side in one launch. A round on such a graph is bound by latency, not by the
+// chip's width, so more graphs in flight on fewer CTAs each is what fills the
+// chip; and a graph costs two team barriers instead of a chain of launches that
+// wait for one another's SMs. 53 graphs of 0.1M to 2M entries: 3.6 ms on eight
+// teams against 5.5 on eight streams. Teams and their graphs are planned on the
+// host (plan_teams); a team's CTAs are its share of the entries.
+constexpr int kMaxTeams = 48;
+
+struct Team {
+  u64* slots;     // min slots, root lists and parents, laid out per graph
+  int4* wl0;      // for its largest graph
+  int4* wl1;
+  unsigned wl_cap;
+  int first_graph;
+  int first_cta;
+};
+struct TeamWords {  // zero when the launch starts
+  unsigned bar[4];  // as DevState::bar
+};
+
+struct TeamArgs {
+  const GraphDesc* graphs;      // by team
+  const LearnedChoice* choice;  // learned mode: by graph, for graphs of learned_min entries or more
+  int teams, learned_min;
+  Team team[kMaxTeams + 1];     // the last one holds the ends of the lists
+  DevState* states;             // by team
+  TeamWords* words;
+  const int* nindex;
+  const int* nlist;
+  const int* eweight;
+  unsigned char* inMST;
+  DevState* st;                 // the batch's error word and atomics counter
+  int mode, explicit_thr, split;
+  float quantile;
+  unsigned solo;
+  int min_tiles;
+  int count_atomics;
+};
+
+__global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) k_batch_group(__grid_constant__ const TeamArgs b) {
+  __shared__ GroupSmem sm;
+  __shared__ GroupArgs g;
+  int t = 0;
+  while (t + 1 < b.teams && (int)blockIdx.x >= b.team[t + 1].first_cta) t++;
+  const Team& team = b.team[t];
+  DevState* st = b.states + t;
+  const unsigned ctas = (unsigned)(b.team[t + 1].first_cta - team.first_cta);
+  GridSync sy;
+  sy.init(st, b.words[t].bar, blockIdx.x - (unsigned)team.first_cta, ctas);
+  bool ok = true;
+  const int last = b.team[t + 1].first_graph;
+  for (int i = team.first_graph; i < last; i++) {
+    if (threadIdx.x == 0) {
+      const GraphDesc d = b.graphs[i];
+      g.nodes = d.nodes;
+      g.edges = d.edges;
+      g.nindex = b.nindex + d.nindex_off;
+      g.nlist = b.nlist + d.edge_off;
+      g.eweight = b.eweight + d.edge_off;
+      g.inMST = b.inMST + d.edge_off;
+      g.minv = team.slots;
+      g.roots0 = reinterpret_cast<int*>(team.slots + d.nodes);
+      g.roots1 = g.roots0 + d.nodes;
+      g.parent = g.roots1 + d.nodes;
+      g.wl0 = team.wl0;
+      g.wl1 = team.wl1;
+      g.wl_cap = team.wl_cap;
+      g.chunk = min(256u, (team.wl_cap - (unsigned)d.edges) / ctas);
+      if (g.chunk < 128) g.chunk = 0;  // a warp may append 128 entries at once
+      g.st = st;
+      g.mode = b.mode == ECL_THRESH_LEARNED && d.edges < b.learned_min ? (int)ECL_THRESH_HEURISTIC : b.mode;
+      g.explicit_thr = b.explicit_thr;
+      g.split = b.split;
+      g.quantile = b.quantile;
+      g.solo = b.solo;
+      g.min_tiles = b.min_tiles;
+      g.count_atomics = b.count_atomics;
+    }
+    if (sy.rank == 0) {  // a clear control block
+      for (int k = threadIdx.x; k < (int)(sizeof(DevState) / sizeof(unsigned)); k += kGroupThreads)
+        reinterpret_cast<unsigned*>(st)[k] = 0;
+      __syncthreads();
+      if (threadIdx.x == 0 && g.mode == ECL_THRESH_LEARNED) {
+        const LearnedChoice c = b.choice[i];
+        st->threshold = c.threshold;
+        st->filtered = c.filtered;
+      }
+    }
+    if (!(ok = sy.sync())) break;
+    if (!(ok = group_solve(g, sy, sm) && sy.sync())) break;
+    if (sy.rank == 0 && threadIdx.x == 0) {
+      if (st->error) atomicOr(&b.st->error, st->error);
+      if (b.count_atomics && st->atomics) atomicAdd(&b.st->atomics, st->atomics);
+    }
+    __syncthreads();  // before the control block is cleared again
+  }
+  if (!ok && threadIdx.x == 0) atomicOr(&b.st->error, kErrTimeout);
 }
 
 }  // namespace ecl

@@ -166,27 +166,21 @@ __host__ __device__ __forceinline__ float heuristic_log2_quantile(int n, int m) 
   return log2f((float)(idx + 1) / 21.f);
 }
 
-// Decode the network output into the solve's control block. Output 0 is the
-// log2 quantile relative to the reference heuristic's; output 1 the log2
-// degree split.
-// One CTA of kH threads: thread j computes hidden unit j of each layer. The
-// decoded quantile selects the light-phase threshold from the sorted weight
-// sample of the feature pass.
-__global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sorted, int n, int m,
-                            ecl::DevState* st, float* feat_out, int lists) {
-  // the whole parameter blob (21 KB) is staged in shared memory first, so the
-  // layers read it at shared-memory latency instead of one global load per
-  // multiply-add
-  __shared__ float p[kParams];
-  __shared__ float fx[kIn], xs[kIn], h1[kH], h2[kH], y[kOut];
+// A solve's schedule from the network's output: output 0 is the log2 quantile
+// relative to the reference heuristic's, output 1 the log2 degree split. The
+// quantile selects the light-phase threshold from the sorted weight sample.
+struct Schedule {
+  float quantile;
+  int threshold, filtered, split;
+};
+
+// One CTA of at least kH threads: thread j computes hidden unit j of each
+// layer, with the parameters (p) in shared memory and f the raw features.
+// Thread 0 gets the schedule.
+__device__ Schedule mlp_schedule(const float* p, const float* f, int n, int m, const int* sorted) {
+  __shared__ float xs[kIn], h1[kH], h2[kH], y[kOut];
   const int j = threadIdx.x;
-  for (int i = j; i < kParams; i += blockDim.x) p[i] = __ldg(pg + i);
-  if (j == 0) compute_features(n, m, acc, sorted, fx);
-  __syncthreads();
-  if (j < kIn) {
-    feat_out[j] = fx[j];  // kept for ecl_mst_ctx_learned_features
-    xs[j] = (fx[j] - p[kOffMean + j]) / p[kOffStd + j];
-  }
+  if (j < kIn) xs[j] = (f[j] - p[kOffMean + j]) / p[kOffStd + j];
   __syncthreads();
   if (j < kH) {
     float a = p[kOffB1 + j];
@@ -206,22 +200,45 @@ __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sort
     y[j] = a;
   }
   __syncthreads();
-  if (j != 0) return;
+  Schedule r{};
+  if (j != 0) return r;
   // output 0 (+ the heuristic's log2 quantile) at or above log2(0.8) means
   // "no filter": a light phase holding 80 % of the entries or more is not
   // worth a second phase (measured on the held-out sweeps)
   const float lq = fminf(fmaxf(heuristic_log2_quantile(n, m) + y[0], -10.f), 0.f);
-  const float q = lq >= kNoFilterLog2Q ? 1.0f : exp2f(lq);
-  st->quantile = q;
-  if (q < 1.0f) {
-    int idx = (int)(q * (float)(kSample - 1));
+  r.quantile = lq >= kNoFilterLog2Q ? 1.0f : exp2f(lq);
+  r.threshold = 0x7fffffff;
+  if (r.quantile < 1.0f) {
+    int idx = (int)(r.quantile * (float)(kSample - 1));
     idx = idx < 0 ? 0 : (idx > kSample - 1 ? kSample - 1 : idx);
-    st->filtered = 1;
-    st->threshold = sorted[idx];
-  } else {
-    st->filtered = 0;
-    st->threshold = 0x7fffffff;
+    r.filtered = 1;
+    r.threshold = sorted[idx];
   }
+  // output 1: log2 of the degree split, in [1, 6]
+  r.split = 1 << (int)lrintf(fminf(fmaxf(y[1], 1.f), 6.f));
+  return r;
+}
+
+// The solve's schedule into its control block, from the feature pass.
+__global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sorted, int n, int m,
+                            ecl::DevState* st, float* feat_out, int lists) {
+  // the whole parameter blob (21 KB) is staged in shared memory first, so the
+  // layers read it at shared-memory latency instead of one global load per
+  // multiply-add
+  __shared__ float p[kParams];
+  __shared__ float fx[kIn];
+  const int j = threadIdx.x;
+  for (int i = j; i < kParams; i += blockDim.x) p[i] = __ldg(pg + i);
+  if (j == 0) compute_features(n, m, acc, sorted, fx);
+  __syncthreads();
+  if (j < kIn) feat_out[j] = fx[j];  // kept for ecl_mst_ctx_learned_features
+  const Schedule r = mlp_schedule(p, fx, n, m, sorted);
+  if (j != 0) return;
+  st->quantile = r.quantile;
+  st->filtered = r.filtered;
+  st->threshold = r.threshold;
+  st->learned_split = r.split;
+  st->split = r.split;  // read by the scans (k_prep leaves it alone in this mode)
   // the lists' split weights, from the same sorted sample (read as unsigned:
   // negative weights come after the others)
   st->split_light = 0xffffffffu;
@@ -235,9 +252,9 @@ __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sort
       }
       return lo;
     };
-    const int neg = count_le(-1), light = count_le(st->threshold);
+    const int neg = count_le(-1), light = count_le(r.threshold);
     float r0, r1;
-    ecl::split_ranks(n, m, st->filtered, (float)light / kSample, &r0, &r1);
+    ecl::split_ranks(n, m, r.filtered, (float)light / kSample, &r0, &r1);
     auto ranked = [&](float r) { return (unsigned)sorted[((int)(r * kSample) + neg) % kSample]; };
     if (r0 < 1.f) st->split_light = ranked(r0);
     if (r1 < 1.f) {
@@ -245,9 +262,42 @@ __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sort
       st->mid = 1;
     }
   }
-  // output 1: log2 of the degree split, in [1, 6]
-  st->learned_split = 1 << (int)lrintf(fminf(fmaxf(y[1], 1.f), 6.f));
-  st->split = st->learned_split;  // read by the scans (k_prep leaves it alone in this mode)
+}
+
+// The degree statistics of a batch's graphs of at least `least` entries:
+// gridDim.x CTAs to each graph (blockIdx.y).
+__global__ void __launch_bounds__(kFeatThreads) k_batch_degrees(const ecl::GraphDesc* graphs, int least,
+                                                                 const int* nindex, FeatAcc* acc) {
+  const ecl::GraphDesc d = graphs[blockIdx.y];
+  if (d.edges < least) return;
+  const int* rows = nindex + d.nindex_off;
+  FeatPart fp;
+  const int stride = gridDim.x * kFeatThreads;
+  for (int v = blockIdx.x * kFeatThreads + threadIdx.x; v < d.nodes; v += stride) {
+    const int b = __ldg(rows + v), e = __ldg(rows + v + 1);
+    fp.add(e > b ? (unsigned)(e - b) : 0u);
+  }
+  fp.fold<kFeatThreads>(acc + blockIdx.y);
+}
+
+// And their schedules: one CTA samples and sorts a graph's weights and runs
+// the network.
+__global__ void __launch_bounds__(kFeatThreads) k_batch_schedule(const float* pg, const ecl::GraphDesc* graphs,
+                                                                  int least, const int* eweight, const FeatAcc* acc,
+                                                                  ecl::LearnedChoice* choice) {
+  extern __shared__ float batch_smem[];  // parameters, then the sorted sample
+  __shared__ float fx[kIn];
+  float* p = batch_smem;
+  int* sorted = reinterpret_cast<int*>(batch_smem + kParams);
+  const ecl::GraphDesc d = graphs[blockIdx.x];
+  if (d.edges < least) return;
+  for (int i = threadIdx.x; i < kParams; i += kFeatThreads) p[i] = __ldg(pg + i);
+  sort_sample(eweight + d.edge_off, d.edges, sorted);
+  __syncthreads();
+  if (threadIdx.x == 0) compute_features(d.nodes, d.edges, acc + blockIdx.x, sorted, fx);
+  __syncthreads();
+  const Schedule r = mlp_schedule(p, fx, d.nodes, d.edges, sorted);
+  if (threadIdx.x == 0) choice[blockIdx.x] = ecl::LearnedChoice{r.threshold, r.filtered};
 }
 
 // Full-batch mean-squared-error loss and gradient of the trainable
@@ -424,6 +474,36 @@ int ecl_learned_apply(ecl_mst_ctx* c, const ecl_graph* g, cudaStream_t s, void* 
   if (r) return r;
   k_mlp_apply<<<1, 256, 0, s>>>(d_params, (const FeatAcc*)d_acc, d_sample, g->nodes, g->edges,
                                (ecl::DevState*)st, d_feat, lists);
+  ML_TRY(cudaGetLastError());
+  return ECL_OK;
+}
+
+// Opt the batch's schedule kernel into its shared memory (once per device).
+int ecl_learned_batch_prepare() {
+  return cuda_status(cudaFuncSetAttribute(k_batch_schedule, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(kParams * sizeof(float) + kSample * sizeof(int))));
+}
+
+// The learned schedules of `count` graphs (device descriptors) of at least
+// `least` entries, with the weights uploaded to c: choice[i] for graph i. The
+// statistics `acc` hold one entry per graph. Two launches on stream s.
+int ecl_learned_batch(ecl_mst_ctx* c, const ecl::GraphDesc* graphs, int count, int least, const int* nindex,
+                      const int* eweight, ecl::FeatAcc* acc, ecl::LearnedChoice* choice, cudaStream_t s) {
+  float *d_params, *d_feat;
+  void* d_acc;
+  int* d_sample;
+  unsigned* version;
+  int sms = 0;
+  int r = ecl_ctx_learned_buffers(c, &d_params, &d_feat, &d_acc, &d_sample, &version, &sms);
+  if (r) return r;
+  ML_TRY(cudaMemsetAsync(acc, 0, (size_t)count * sizeof(FeatAcc), s));
+  for (int i = 0; i < count; i += 65535) {  // the limit of gridDim.y
+    const int part = std::min(count - i, 65535);
+    k_batch_degrees<<<dim3(std::max(1, 4 * sms / part), part), kFeatThreads, 0, s>>>(graphs + i, least, nindex, acc + i);
+    ML_TRY(cudaGetLastError());
+  }
+  k_batch_schedule<<<count, kFeatThreads, kParams * sizeof(float) + kSample * sizeof(int), s>>>(
+      d_params, graphs, least, eweight, acc, choice);
   ML_TRY(cudaGetLastError());
   return ECL_OK;
 }

@@ -100,6 +100,17 @@ struct BorState {
   int skip;    // the tree that offers nothing, -1 = none
 };
 
+// One graph of a batch: where its rows and entries start in the batch's arrays.
+struct GraphDesc {
+  long long nindex_off, edge_off;
+  int nodes, edges;
+};
+
+// The learned schedule's choice for one graph of a batch.
+struct LearnedChoice {
+  int threshold, filtered;
+};
+
 // The worklists a solve's scans build, in the order their rounds run. The light
 // phase's entries may be split by weight into two lists, and the light scan may
 // set aside the lightest of the heavy phase's: rounds on a short list of the
@@ -115,7 +126,7 @@ struct ListCount {
 };
 
 // Control block of one solve, zeroed before every solve.
-struct DevState {
+struct alignas(128) DevState {
   int threshold;       // light phase keeps w <= threshold
   int filtered;        // 1 = light + heavy phase, 0 = one unfiltered phase
   int split;           // degree split between the thread and the chunk tier
@@ -144,9 +155,7 @@ struct DevState {
   unsigned seg_off[kMaxRoundCtas];
   unsigned root_cnt[4][3];  // [list][pass % 3] = live roots a roots pass kept
   BorState resume;          // where the cluster kernel goes on with the phase
-  unsigned bar[4];          // GridSync counters: k_round's by list; k_group's
-  unsigned gate;            // the last gate opened (GridSync::regroup)
-  unsigned gate_target;
+  unsigned bar[4];          // GridSync: k_round's counters by list; k_group's counter and gate
   unsigned graph;           // batch: the graph the cluster works on
   int giant;                // the light phase's largest tree (by a vote of sampled vertices)
 };

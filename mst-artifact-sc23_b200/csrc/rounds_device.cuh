@@ -120,23 +120,24 @@ __device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Barrier among the first `active` CTAs of a cooperative launch: one release
-// add per CTA to a counter that only grows, and an acquire poll of the same
-// counter by one thread; the other threads are ordered through the CTA
-// barriers on both sides. (A counter that the last CTA resets before it
-// releases a generation word took 1.85 us on 32 to 296 CTAs.) The wait is
-// bounded (kErrTimeout, and every later barrier then returns false).
+// Barrier among the first `active` of the `ctas` CTAs of a cooperative launch,
+// or of one of its teams: one release add per CTA to a counter that only
+// grows, and an acquire poll of the same counter by one thread; the other
+// threads are ordered through the CTA barriers on both sides. (A counter that
+// the last CTA resets before it releases a generation word took 1.85 us on 32
+// to 296 CTAs.) The wait is bounded (kErrTimeout, and every later barrier then
+// returns false).
 struct GridSync {
   static constexpr bool kGrid = true;
   DevState* st;
-  unsigned* word;  // zero when the launch starts
-  unsigned rank, active, target;
-  __device__ __forceinline__ void init(DevState* s, unsigned* counter) {
+  unsigned* word;  // the counter; regroup: [1] the last gate opened, [2] the barrier count there; zero at first
+  unsigned rank, ctas, active, target, gates;
+  __device__ __forceinline__ void init(DevState* s, unsigned* words, unsigned r, unsigned n) {
     st = s;
-    word = counter;
-    rank = blockIdx.x;
-    active = gridDim.x;
-    target = 0;
+    word = words;
+    rank = r;
+    active = ctas = n;
+    target = gates = 0;
   }
   __device__ __forceinline__ bool poll(const unsigned* p, unsigned at_least, bool nap) {
     u64 t0 = 0;
@@ -162,23 +163,24 @@ struct GridSync {
     }
     return __syncthreads_and(ok);
   }
-  // All CTAs of the launch again, after rounds some of them `left`: those wait
-  // until the first CTA, done with the rounds, opens gate number `gate`, and
-  // take over its count of the barriers.
-  __device__ __forceinline__ bool regroup(bool left, unsigned gate) {
+  // All CTAs again, after rounds some of them `left`: those wait until the
+  // first CTA, done with the rounds, opens the next gate, and take over its
+  // count of the barriers.
+  __device__ __forceinline__ bool regroup(bool left) {
     bool ok = true;
+    gates++;
     __syncthreads();
     if (threadIdx.x == 0) {
       if (rank == 0) {
-        st->gate_target = target;
-        st_release_gpu(&st->gate, gate);
+        word[2] = target;
+        st_release_gpu(word + 1, gates);
       } else if (left) {
-        ok = poll(&st->gate, gate, true);
+        ok = poll(word + 1, gates, true);
       }
     }
-    active = gridDim.x;
+    active = ctas;
     ok = __syncthreads_and(ok);
-    if (left) target = ld_volatile(&st->gate_target);
+    if (left) target = ld_volatile(word + 2);
     return ok;
   }
 };
@@ -201,7 +203,7 @@ struct ClusterSync {
     return true;
   }
   // The whole cluster again: the CTAs that left the rounds wait at its barrier.
-  __device__ __forceinline__ bool regroup(bool, unsigned) {
+  __device__ __forceinline__ bool regroup(bool) {
     active = ctas;
     return sync();
   }
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(kBorThreads, kBorBlocks) k_round(BorArgs a) {
   b.first = 1;
   b.skip = first ? -1 : st->giant;
   GridSync sy;
-  sy.init(st, &st->bar[a.list]);
+  sy.init(st, &st->bar[a.list], blockIdx.x, gridDim.x);
   bor_smem_init(s);
   __syncthreads();
   const bool stamp = sy.rank == 0 && threadIdx.x == 0;
