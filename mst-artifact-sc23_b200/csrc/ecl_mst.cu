@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <utility>
 
 #include "ecl_mst.h"
 #include "internal.h"
@@ -267,14 +268,13 @@ namespace {
 // overflows them. Both carry slack for the unused tails of the scan warps'
 // slot chunks.
 int alloc_worklists(ecl_mst_ctx* c, bool full) {
-  cudaFree(c->wl[0]);
-  cudaFree(c->wl[1]);
+  cudaFree(c->wl[0]);  // holds both
   c->wl[0] = c->wl[1] = nullptr;
   const int64_t keep = full ? c->max_edges : c->max_edges / 2;
   c->wl_cap = (unsigned)std::max<int64_t>(keep + std::min<int64_t>(c->max_edges, kWlSlack), 1);
   c->wl_full = full;
-  for (int i = 0; i < 2; i++)
-    ECL_CUDA_TRY(cudaMalloc(&c->wl[i], (size_t)c->wl_cap * sizeof(int4)));
+  ECL_CUDA_TRY(cudaMalloc(&c->wl[0], 2 * (size_t)c->wl_cap * sizeof(int4)));
+  c->wl[1] = c->wl[0] + c->wl_cap;
   return ECL_OK;
 }
 
@@ -287,8 +287,8 @@ extern "C" void ecl_default_opts(mst_opts* o) {
   o->quantile = 1.0f;
 }
 
-extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edges,
-                                  ecl_mst_ctx** out) {
+// `full`: worklists for any input from the start.
+static int ctx_create(int device, int64_t max_nodes, int64_t max_edges, bool full, ecl_mst_ctx** out) {
   if (!out || max_nodes < 1 || max_edges < 0 || max_nodes > INT32_MAX || max_edges > INT32_MAX)
     return ECL_ERR_INVALID_ARG;
   *out = nullptr;
@@ -306,30 +306,46 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
     ecl_mst_ctx_destroy(c);
     return s;
   };
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return fail(ECL_ERR_CUDA);
-  if (!prop.cooperativeLaunch) return fail(ECL_ERR_UNSUPPORTED);
-  c->sm_count = prop.multiProcessorCount;
+  int coop = 0, persist = 0, window = 0;
+  for (const auto& q : {std::make_pair(&coop, cudaDevAttrCooperativeLaunch),
+                        std::make_pair(&c->sm_count, cudaDevAttrMultiProcessorCount),
+                        std::make_pair(&persist, cudaDevAttrMaxPersistingL2CacheSize),
+                        std::make_pair(&window, cudaDevAttrMaxAccessPolicyWindowSize)})
+    if ((st = cuda_status(cudaDeviceGetAttribute(q.first, q.second, device)))) return fail(st);
+  if (!coop) return fail(ECL_ERR_UNSUPPORTED);
   if ((st = cuda_status(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)))) return fail(st);
   if ((st = cuda_status(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking)))) return fail(st);
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)))) return fail(st);
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming)))) return fail(st);
   if ((st = cuda_status(cudaEventCreateWithFlags(&c->prep_done, cudaEventDisableTiming)))) return fail(st);
-  const size_t slot_bytes = (size_t)max_nodes * (2 * sizeof(u64) + sizeof(int));
-  if ((st = cuda_status(cudaMalloc(&c->slots, slot_bytes)))) return fail(st);
-  c->l2_persist_max = prop.persistingL2CacheMaxSize > 0 ? (size_t)prop.persistingL2CacheMaxSize : 0;
-  c->l2_window_max = prop.accessPolicyMaxWindowSize > 0 ? (size_t)prop.accessPolicyMaxWindowSize : 0;
-  if ((st = alloc_worklists(c, false))) return fail(st);
+  c->l2_persist_max = (size_t)std::max(persist, 0);
+  c->l2_window_max = (size_t)std::max(window, 0);
   c->first_v_cap = (int)first_v_entries(max_edges);
-  if ((st = cuda_status(cudaMalloc(&c->first_v, (size_t)c->first_v_cap * sizeof(int))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->tree_bits, tree_bits_bytes(max_nodes))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->st, sizeof(DevState))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->ml_params, ECL_MLP_PARAMS * sizeof(float))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->ml_feat, ECL_MLP_INPUTS * sizeof(float))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->ml_acc, sizeof(FeatAcc))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->ml_sample, 4096 * sizeof(int))))) return fail(st);
-  if ((st = cuda_status(cudaHostAlloc(&c->st_host, sizeof(DevState), cudaHostAllocDefault))))
-    return fail(st);
+  // one allocation (its pointer is c->slots) for everything but the worklists,
+  // which may grow: an allocation and its release take 0.7 ms together
+  size_t bytes = 0;
+  auto carve = [&](size_t size) {
+    const size_t at = bytes;
+    bytes += (size + 255) & ~(size_t)255;
+    return at;
+  };
+  carve((size_t)max_nodes * (2 * sizeof(u64) + sizeof(int)));
+  const size_t first_v = carve((size_t)c->first_v_cap * sizeof(int)), bits = carve(tree_bits_bytes(max_nodes));
+  const size_t state = carve(sizeof(DevState)), params = carve(ECL_MLP_PARAMS * sizeof(float));
+  const size_t feat = carve(ECL_MLP_INPUTS * sizeof(float)), acc = carve(sizeof(FeatAcc));
+  const size_t sample = carve(4096 * sizeof(int));
+  if ((st = cuda_status(cudaMalloc(&c->slots, bytes)))) return fail(st);
+  unsigned char* base = static_cast<unsigned char*>(c->slots);
+  c->first_v = reinterpret_cast<int*>(base + first_v);
+  c->tree_bits = reinterpret_cast<unsigned*>(base + bits);
+  c->st = reinterpret_cast<DevState*>(base + state);
+  c->ml_params = reinterpret_cast<float*>(base + params);
+  c->ml_feat = reinterpret_cast<float*>(base + feat);
+  c->ml_acc = base + acc;
+  c->ml_sample = reinterpret_cast<int*>(base + sample);
+  if ((st = alloc_worklists(c, full))) return fail(st);
+  c->st_host = new (std::nothrow) DevState();  // not pinned: that takes 2 ms, a copy to it 10 us
+  if (!c->st_host) return fail(ECL_ERR_ALLOC);
   for (auto& e : c->ev)
     if ((st = cuda_status(cudaEventCreate(&e)))) return fail(st);
   // every CTA of a round pass writes one segment of the round's output list
@@ -345,6 +361,11 @@ extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edg
   return ECL_OK;
 }
 
+extern "C" int ecl_mst_ctx_create(int device, int64_t max_nodes, int64_t max_edges,
+                                  ecl_mst_ctx** out) {
+  return ctx_create(device, max_nodes, max_edges, false, out);
+}
+
 extern "C" void ecl_mst_ctx_destroy(ecl_mst_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
@@ -353,28 +374,14 @@ extern "C" void ecl_mst_ctx_destroy(ecl_mst_ctx* c) {
     cudaCtxResetPersistingL2Cache();
     cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, c->l2_limit_prev);
   }
-  cudaFree(c->slots);
-  cudaFree(c->wl[0]);
-  cudaFree(c->wl[1]);
-  cudaFree(c->first_v);
-  cudaFree(c->tree_bits);
+  cudaFree(c->slots);     // and what lies behind the slots
+  cudaFree(c->wl[0]);     // both lists
   cudaFree(c->slist);
-  cudaFree(c->ml_params);
-  cudaFree(c->ml_feat);
-  cudaFree(c->ml_acc);
-  cudaFree(c->ml_sample);
-  cudaFree(c->st);
-  cudaFreeHost(c->st_host);
-  cudaFree(c->d_nindex);
-  cudaFree(c->d_nlist);
-  cudaFree(c->d_eweight);
-  cudaFree(c->d_inMST);
+  delete c->st_host;
+  cudaFree(c->d_nindex);  // all four arrays
   if (c->cin) cudaStreamSynchronize(c->cin);
   if (c->cout) cudaStreamSynchronize(c->cout);
   cudaFree(c->hs[1].nindex);
-  cudaFree(c->hs[1].nlist);
-  cudaFree(c->hs[1].eweight);
-  cudaFree(c->hs[1].inMST);
   cudaFree(c->sticky);
   for (auto& h : c->hs)
     for (cudaEvent_t e : {h.in_done, h.solved, h.out_done})
@@ -1063,11 +1070,14 @@ namespace {
 // Device CSR and inMST buffers for host-buffer solves, allocated on first use.
 int host_buffers(ecl_mst_ctx* c, int** ni, int** nl, int** ew, unsigned char** out) {
   if (*ni) return ECL_OK;
-  const size_t nb = ((size_t)c->max_nodes + 1) * 4, eb = (size_t)std::max<int64_t>(c->max_edges, 1) * 4;
-  ECL_CUDA_TRY(cudaMalloc(ni, nb));
-  ECL_CUDA_TRY(cudaMalloc(nl, eb));
-  ECL_CUDA_TRY(cudaMalloc(ew, eb));
-  ECL_CUDA_TRY(cudaMalloc(out, eb / 4));
+  // one allocation, whose pointer is *ni
+  auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t m = (size_t)std::max<int64_t>(c->max_edges, 1);
+  const size_t nb = align(((size_t)c->max_nodes + 1) * 4), eb = align(m * 4);
+  ECL_CUDA_TRY(cudaMalloc(ni, nb + 2 * eb + align(m)));
+  *nl = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(*ni) + nb);
+  *ew = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(*nl) + eb);
+  *out = reinterpret_cast<unsigned char*>(*ew) + eb;
   return ECL_OK;
 }
 
@@ -1516,13 +1526,7 @@ struct ecl_batch_ctx {
 // so its lists hold every entry of any input.
 static int batch_big_ctx(ecl_batch_ctx* c, int k) {
   if (c->big[k]) return ECL_OK;
-  int st = ecl_mst_ctx_create(c->device, c->max_nodes, std::max<int64_t>(c->max_edges, 1), &c->big[k]);
-  if (!st) st = alloc_worklists(c->big[k], true);
-  if (st) {
-    ecl_mst_ctx_destroy(c->big[k]);
-    c->big[k] = nullptr;
-  }
-  return st;
+  return ctx_create(c->device, c->max_nodes, std::max<int64_t>(c->max_edges, 1), true, &c->big[k]);
 }
 
 extern "C" void ecl_batch_ctx_destroy(ecl_batch_ctx* c) {

@@ -375,17 +375,36 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
   const int64_t total = 2 * pairs;
   const int bits = id_bits(nodes);
   const bool given = rule == ECL_WEIGHTS_GIVEN;
-  Scratch sc(s);
-  uint64_t *keys = nullptr, *keys_alt = nullptr;
-  uint32_t *vals = nullptr, *vals_alt = nullptr, *pos = nullptr;
-  unsigned long long* counters = nullptr;  // [0] dropped keys, [1] bad-id flag
-  PP_CHECK(sc.get(&counters, 2));
-  PP_CHECK(sc.get(&keys, total));
-  PP_CHECK(sc.get(&keys_alt, total));
-  if (given) {
-    PP_CHECK(sc.get(&vals, total));
-    PP_CHECK(sc.get(&vals_alt, total));
+  // all scratch in one piece: the pool starts empty, and every piece it has to
+  // map takes time (5M pairs with weights 6.3 ms, 6.65 in eight pieces)
+  size_t sort_bytes = 0, scan_bytes = 0;
+  if (total > 0) {
+    cub::DoubleBuffer<uint64_t> kb(nullptr, nullptr);
+    cub::DoubleBuffer<uint32_t> vb(nullptr, nullptr);
+    if (given) PP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kb, vb, (int)total, 0, 2 * bits, s));
+    else PP_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, kb, (int)total, 0, 2 * bits, s));
+    PP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)(total + 1), s));
   }
+  size_t bytes = 0;
+  auto carve = [&](size_t size) {
+    const size_t at = bytes;
+    bytes += (size + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t at_counters = carve(2 * sizeof(unsigned long long)), at_keys = carve((size_t)total * 8);
+  const size_t at_keys_alt = carve((size_t)total * 8), at_vals = carve(given ? (size_t)total * 4 : 0);
+  const size_t at_vals_alt = carve(given ? (size_t)total * 4 : 0), at_pos = carve(((size_t)total + 1) * 4);
+  const size_t at_tmp = carve(std::max(sort_bytes, scan_bytes));
+  Scratch sc(s);
+  char* base = nullptr;
+  PP_CHECK(sc.get(&base, bytes));
+  auto* counters = reinterpret_cast<unsigned long long*>(base + at_counters);  // [0] dropped keys, [1] bad-id flag
+  auto* keys = reinterpret_cast<uint64_t*>(base + at_keys);
+  auto* keys_alt = reinterpret_cast<uint64_t*>(base + at_keys_alt);
+  auto* vals = given ? reinterpret_cast<uint32_t*>(base + at_vals) : nullptr;
+  auto* vals_alt = given ? reinterpret_cast<uint32_t*>(base + at_vals_alt) : nullptr;
+  auto* pos = reinterpret_cast<uint32_t*>(base + at_pos);
+  char* tmp = base + at_tmp;
   PP_TRY(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s));
   int64_t valid = 0;
   uint64_t* spare = keys_alt;  // the sort's other buffer, free after the sort
@@ -397,17 +416,11 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
     PP_TRY(cudaGetLastError());
     cub::DoubleBuffer<uint64_t> kb(keys, keys_alt);
     cub::DoubleBuffer<uint32_t> vb(vals, vals_alt);
-    size_t tmp_bytes = 0;
-    char* tmp = nullptr;
     if (given) {
-      PP_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, kb, vb, (int)total, 0, 2 * bits, s));
-      PP_CHECK(sc.get(&tmp, tmp_bytes));
-      PP_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, (int)total, 0, 2 * bits, s));
+      PP_TRY(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, kb, vb, (int)total, 0, 2 * bits, s));
       vals = vb.Current();
     } else {
-      PP_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, kb, (int)total, 0, 2 * bits, s));
-      PP_CHECK(sc.get(&tmp, tmp_bytes));
-      PP_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, kb, (int)total, 0, 2 * bits, s));
+      PP_TRY(cub::DeviceRadixSort::SortKeys(tmp, sort_bytes, kb, (int)total, 0, 2 * bits, s));
     }
     keys = kb.Current();
     spare = kb.Alternate();
@@ -421,14 +434,9 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
   if (valid > 0) {
     // run-head flags in the spare sort buffer ((valid + 1) * 4 <= total * 8 bytes)
     uint32_t* flags = reinterpret_cast<uint32_t*>(spare);
-    PP_CHECK(sc.get(&pos, (size_t)valid + 1));
     k_run_heads<<<blocks_for(valid + 1), kPT, 0, s>>>(valid, keys, flags);
     PP_TRY(cudaGetLastError());
-    size_t tmp_bytes = 0;
-    char* tmp = nullptr;
-    PP_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flags, pos, (int)(valid + 1), s));
-    PP_CHECK(sc.get(&tmp, tmp_bytes));
-    PP_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, pos, (int)(valid + 1), s));
+    PP_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, flags, pos, (int)(valid + 1), s));
     uint32_t hm = 0;
     PP_TRY(cudaMemcpyAsync(&hm, pos + valid, sizeof(hm), cudaMemcpyDeviceToHost, s));
     PP_TRY(cudaStreamSynchronize(s));
