@@ -391,9 +391,9 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
     bytes += (size + 255) & ~(size_t)255;
     return at;
   };
-  const size_t at_counters = carve(2 * sizeof(unsigned long long)), at_keys = carve((size_t)total * 8);
-  const size_t at_keys_alt = carve((size_t)total * 8), at_vals = carve(given ? (size_t)total * 4 : 0);
-  const size_t at_vals_alt = carve(given ? (size_t)total * 4 : 0), at_pos = carve(((size_t)total + 1) * 4);
+  const size_t at_counters = carve(2 * sizeof(unsigned long long)), at_keys = carve(((size_t)total + 1) * 8);
+  const size_t at_keys_alt = carve(((size_t)total + 1) * 8), at_vals = carve(given ? (size_t)total * 4 : 0);
+  const size_t at_vals_alt = carve(given ? (size_t)total * 4 : 0);
   const size_t at_tmp = carve(std::max(sort_bytes, scan_bytes));
   Scratch sc(s);
   char* base = nullptr;
@@ -403,7 +403,7 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
   auto* keys_alt = reinterpret_cast<uint64_t*>(base + at_keys_alt);
   auto* vals = given ? reinterpret_cast<uint32_t*>(base + at_vals) : nullptr;
   auto* vals_alt = given ? reinterpret_cast<uint32_t*>(base + at_vals_alt) : nullptr;
-  auto* pos = reinterpret_cast<uint32_t*>(base + at_pos);
+  uint32_t* pos = nullptr;
   char* tmp = base + at_tmp;
   PP_TRY(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s));
   int64_t valid = 0;
@@ -432,8 +432,9 @@ int build_csr(int32_t nodes, int64_t pairs, const int32_t* u, const int32_t* v, 
   }
   int32_t m = 0;
   if (valid > 0) {
-    // run-head flags in the spare sort buffer ((valid + 1) * 4 <= total * 8 bytes)
+    // run-head flags and their sums in the spare sort buffer (2 * 4 * (valid + 1) bytes)
     uint32_t* flags = reinterpret_cast<uint32_t*>(spare);
+    pos = flags + (valid + 1);
     k_run_heads<<<blocks_for(valid + 1), kPT, 0, s>>>(valid, keys, flags);
     PP_TRY(cudaGetLastError());
     PP_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, flags, pos, (int)(valid + 1), s));
