@@ -238,28 +238,27 @@ typedef struct mst_opts {
   int32_t threshold;      /* ECL_THRESH_EXPLICIT: edges with w <= threshold    */
                           /* form the first (light) phase                      */
   float quantile;         /* ECL_THRESH_QUANTILE, in [0,1]; >= 1 disables      */
-  int32_t degree_split;   /* thread/cooperative split of the light CSR scan:   */
-                          /* each thread takes E consecutive entries, E = 4    */
-                          /* for split <= 4, 8 for split <= 8, else 16; rows   */
-                          /* shorter than E stay in one thread, longer rows    */
-                          /* are spread over threads/warps; 0 = default (8).   */
-                          /* The heavy scan always takes E = 4                 */
-  int32_t round_min_tiles; /* the round kernel keeps one CTA per this many   */
-                          /* 512-entry tiles of a round's worklist: CTAs       */
+  int32_t degree_split;   /* the reference's thread/warp split by row degree;  */
+                          /* reported in the statistics, 0 = default (8): the  */
+                          /* scans' warps work by entries and need none        */
+  int32_t round_min_tiles; /* the round kernels keep one CTA per this many   */
+                          /* 1024-entry tiles of a round's worklist: CTAs      */
                           /* beyond it leave the launch as the rounds shrink,  */
                           /* and its grid barriers wait for the rest only;     */
                           /* 0 = default (1), < 0 = keep every CTA             */
-  int32_t ctas_per_sm;    /* round-kernel CTAs per SM, 0 = as many as fit      */
+  int32_t ctas_per_sm;    /* most CTAs per SM of a graph's round kernel, 0 =   */
+                          /* as many as fit (and one cluster for a small one)  */
   int32_t small_tail;     /* worklist size at which one CTA finishes the      */
                           /* rounds alone; 0 = default, < 0 = never            */
   int32_t flags;          /* ECL_FLAG_*                                        */
   int32_t batch_small_edges; /* batched mode: graphs with at most this many   */
-                          /* CSR entries (and fitting the per-CTA scratch) are */
-                          /* solved one per CTA by the persistent kernel;      */
-                          /* 0 = the context's per-CTA capacity                */
+                          /* CSR entries (and fitting the scratch) are solved  */
+                          /* by one cluster each, in persistent launches;      */
+                          /* 0 = the context's capacity                        */
   int32_t batch_large_streams; /* batched mode: the other graphs are solved on */
                           /* this many concurrent streams (1..8), each with    */
-                          /* its own workspace, largest graph first to the     */
+                          /* its own workspace (which teams of CTAs share for  */
+                          /* the mid-size ones), largest graph first to the    */
                           /* least-loaded stream; with more than one, their    */
                           /* round kernels take one CTA per SM unless          */
                           /* ctas_per_sm is set; 0 = default (4); fewer when   */
@@ -275,12 +274,14 @@ void ecl_default_opts(mst_opts* opts);
 typedef struct ecl_mst_stats {
   int32_t threshold;       /* threshold used (INT32_MAX when unfiltered)        */
   int32_t filtered;        /* 1 if two phases ran                               */
-  int32_t degree_split;    /* split used by the light scan                      */
+  int32_t degree_split;    /* the split asked for, or the network's             */
   int32_t rounds[2];       /* Boruvka rounds of the light / heavy phase         */
   int32_t status;          /* device error word (0 = clean)                     */
   int64_t scan_kept[2];    /* worklist entries appended by each scan            */
-  int64_t wl_in[2][ECL_MAX_ROUNDS];  /* worklist slots entering each round (the
-                                        first also holds null padding)       */
+  int64_t wl_in[2][ECL_MAX_ROUNDS];  /* worklist slots entering each round (a
+                                        list's first also holds null padding);
+                                        a phase may run several lists, split by
+                                        weight, one after another            */
   int64_t atomics;         /* guarded atomicMin issued (ECL_FLAG_STATS only)    */
   int64_t forest_edges;    /* number of inMST entries set                       */
   uint64_t forest_weight;  /* sum of eweight over inMST (as verify(), :377)     */
@@ -293,8 +294,9 @@ typedef struct ecl_mst_stats {
    * device clock at the round kernel's barriers:                            */
   float us_scan[2][3];     /* [0]: {features + prep + light scan, features +
                               prep, light scan kernel}; [1]: {flatten + heavy
-                              scan, flatten, heavy scan kernel}                */
-  float us_round[2][ECL_MAX_ROUNDS][2]; /* per round: find/min pass, mark pass  */
+                              scan, flatten (and the rounds of the heavy list
+                              set aside), heavy scan kernel}                   */
+  float us_round[2][ECL_MAX_ROUNDS][2]; /* per round: offer pass, mark + roots  */
   int64_t wl_real[2][ECL_MAX_ROUNDS];   /* entries entering each round without
                                            the scans' null padding            */
 } ecl_mst_stats;
@@ -399,8 +401,8 @@ typedef struct ecl_batch {
 } ecl_batch;
 
 typedef struct ecl_batch_stats {
-  int32_t graphs_small;  /* solved one per CTA in the persistent launch */
-  int32_t graphs_large;  /* solved by the grid-wide engine                */
+  int32_t graphs_small;  /* solved by one cluster each                 */
+  int32_t graphs_large;  /* solved by teams of CTAs or the engines        */
   int32_t status;        /* device error word                             */
   int32_t graph_replay;  /* 1 if the large graphs ran from a CUDA graph     */
   int64_t edges_total;
@@ -410,9 +412,9 @@ typedef struct ecl_batch_stats {
 typedef struct ecl_batch_ctx ecl_batch_ctx;
 
 /* Workspace for batches of up to max_graphs graphs, none larger than
- * (max_graph_nodes, max_graph_edges). small_cap sizes the per-CTA scratch of
- * the persistent kernel (vertices and entries of the largest graph it may
- * take; 0 = 2^19). */
+ * (max_graph_nodes, max_graph_edges). small_cap sizes the scratch of the
+ * cluster kernels (vertices and entries of the largest graph they may take;
+ * 0 = 2^19). */
 int ecl_batch_ctx_create(int device, int32_t max_graphs, int64_t max_graph_nodes,
                          int64_t max_graph_edges, int32_t small_cap,
                          ecl_batch_ctx** out);
@@ -424,8 +426,8 @@ int ecl_mst_run_batch_device(ecl_batch_ctx* ctx, const ecl_batch* batch,
                              uint8_t* d_inMST, const mst_opts* opts, void* stream,
                              ecl_batch_stats* stats);
 
-/* Autotuner: times candidate schedules (per-CTA cutoff, scan entries per
- * thread and, when *base asks for the learned schedule, learned against the
+/* Autotuner: times candidate schedules (small-graph cutoff, degree split
+ * and, when *base asks for the learned schedule, learned against the
  * reference heuristic for the large graphs; then, unless *base sets them,
  * the large graphs' streams and round-kernel CTAs per SM, and the cutoff
  * again with those) on the batch and

@@ -116,7 +116,7 @@ struct ecl_mst_ctx {
   unsigned* tree_bits = nullptr;  // bit v: v lies in the light phase's largest tree
   int first_v_cap = 0;
   DevState* st = nullptr;
-  DevState* st_host = nullptr;  // pinned
+  DevState* st_host = nullptr;  // statistics of the last solve
   int round_grid = 0;  // most co-resident CTAs of k_round
   int abl_grid = 0;    // the same of k_rounds (ablation variants)
   int group_grid = 0;  // the same of k_group
@@ -2056,7 +2056,7 @@ extern "C" int ecl_batch_autotune(ecl_batch_ctx* c, const ecl_batch* b, uint8_t*
   };
   int st;
   const int cutoffs[] = {c->cap / 8, c->cap / 4, c->cap / 2, c->cap};
-  // 1. per-CTA cutoff, scan entries per lane and schedule. The learned
+  // 1. small-graph cutoff, degree split and schedule. The learned
   //    schedule (large graphs only) is kept only where it beats the
   //    reference heuristic on this batch.
   const int modes[] = {o0.threshold_mode, ECL_THRESH_HEURISTIC};
