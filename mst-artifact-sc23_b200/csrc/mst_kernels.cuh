@@ -169,16 +169,20 @@ struct alignas(128) DevState {
 // latency, 100-150 us (ER 3M, 4.4M light entries: 0.99 ms against 1.06, 1.21 at
 // 0.25 x n; RMAT-18 unfiltered, 3.8M: 0.38 against 0.50; ER 1.2M, 1.7M: 0.66
 // against 0.57).
+//   Beyond L2 (kMidNodes) an entry dropped early saves more: kSplitLightFar
+// (ER 16M 7.21 ms against 7.68, RMAT-25 the same; in L2, RMAT-22 1.42 ms against
+// 1.36).
 //   Heavy entries: list mid takes them up to kSplitHeavy x n entries in all,
 // where the slots and parents of the vertices outgrow L2, so that every entry
 // the heavy scan keeps costs DRAM accesses (ER 16M 7.7 ms against 8.9, RMAT-25
 // 10.8 against 11.7; RMAT-22, in L2, 1.55 against 1.52).
-constexpr float kSplitLight = 0.5f, kSplitHeavy = 2.0f;
+constexpr float kSplitLight = 0.5f, kSplitLightFar = 0.8f, kSplitHeavy = 2.0f;
 constexpr int kSplitMin = 3 << 20;
 constexpr int kMidNodes = 1 << 23;
 __device__ __forceinline__ void split_ranks(int n, int m, int filtered, float light_share, float* rank0, float* rank1) {
   const float half = 0.5f * (float)m;
-  const float f0 = kSplitLight * (float)n / half, f1 = kSplitHeavy * (float)n / half;
+  const float f0 = (n >= kMidNodes ? kSplitLightFar : kSplitLight) * (float)n / half;
+  const float f1 = kSplitHeavy * (float)n / half;
   *rank0 = f0 * 1.5f < light_share && light_share * half >= (float)kSplitMin ? f0 : 2.f;
   *rank1 = filtered && n >= kMidNodes && f1 > 1.3f * light_share && f1 <= 0.4f ? f1 : 2.f;
 }
