@@ -636,6 +636,9 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, Sync& 
       }
     }
     if (stamp) st->root_cnt[a.list][(b.flips + 1) % 3] = 0;  // the next roots pass's counter
+    // Every warp has read its count of the CTA's entries before it is cleared:
+    // the steps' CTA barriers see to that, but steps without a list have none.
+    if (b.first && !all && !rout) __syncthreads();
     if (tid == 0) s.cursor = 0;
     if (!sy.sync()) break;
     if (stamp) st->t_round[ph][2 * b.r - 1] = globaltimer_ns();
