@@ -104,6 +104,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
     }
     int lo, hi;
     warp_rows(g.nindex, n, jw, min(jw + 127, m - 1), lo, hi);
+    const int top = hi;
     while (lo < hi && own > 0) {  // the last row starting at or before j0
       const int mid = lo + ((hi - lo + 1) >> 1);
       if (__ldg(g.nindex + mid) <= j0) lo = mid;
@@ -115,7 +116,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       if (i < own) {
-        while (j0 + i >= end && v < n - 1) end = __ldg(g.nindex + ++v + 1);
+        row_on([&](int r) { return __ldg(g.nindex + r); }, top, j0 + i, v, end);
         bad |= (unsigned)nb[i] >= (unsigned)n;
         // one direction with a valid id (v < nb < n) as one unsigned compare
         if ((unsigned)nb[i] - (unsigned)v - 1u < (unsigned)(n - v - 1) && (KIND == kLight ? w[i] <= thr : w[i] > thr))

@@ -3,6 +3,7 @@
 // Shared by the single-graph engine (ecl_mst.cu) and the batched engine.
 #pragma once
 #include <cuda_runtime.h>
+#include <climits>
 #include <stdint.h>
 
 #include "ecl_mst.h"
@@ -237,6 +238,29 @@ __device__ __forceinline__ int ld_ca(const int* p) {
   int v;
   asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+
+// On from row v, whose entries end at `end`, to the row of entry j, which is at
+// most `top`: first(r) is row r's first entry. A few rows are looked at one by
+// one. A longer run is one of empty rows, of any length, and is bisected: a
+// million isolated vertices between two entries of a thread, walked row by row,
+// took 50 ms a scan.
+constexpr int kRowSteps = 4;
+template <class First>
+__device__ __forceinline__ void row_on(First first, int top, int j, int& v, int& end) {
+  for (int k = 0; j >= end && v < top; k++) {
+    if (k == kRowSteps) {
+      int lo = v + 1, hi = top;  // row v + 1 starts at `end`
+      while (lo < hi) {
+        const int mid = lo + ((hi - lo + 1) >> 1);
+        if (first(mid) <= j) lo = mid;
+        else hi = mid - 1;
+      }
+      v = lo - 1;
+    }
+    v++;
+    end = v < top ? first(v + 1) : INT_MAX;
+  }
 }
 
 // ---- mbarriers and bulk asynchronous copies (cp.async.bulk, no multicast)

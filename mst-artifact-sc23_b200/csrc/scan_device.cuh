@@ -304,14 +304,16 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocks) k_scan_light(ScanAr
           if (slice_at(a, rows, slice, mid_row) <= j0 + at) lo = mid_row;
           else hi = mid_row - 1;
         }
-        int row = lo;
+        auto first = [&](int r) { return slice_at(a, rows, slice, r); };
+        const int top = rows.hi - rows.lo;
+        int row = lo, end = row < top ? first(row + 1) : INT_MAX;
         const int4 y = g == 0 ? nb[0] : g == 1 ? nb[1] : g == 2 ? nb[2] : nb[3];
         const int ends[4] = {y.x, y.y, y.z, y.w};
         int4 e[4];
         unsigned cls = 0xffffu;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          while (row < rows.hi - rows.lo && slice_at(a, rows, slice, row + 1) <= j0 + at + i) row++;
+          row_on(first, top, j0 + at + i, row, end);
           const int v = rows.lo + row;
           e[i] = make_int4(v, ends[i], data[at + i], j0 + at + i);
           const bool on = (mask >> (4 * g + i)) & 1u;
