@@ -42,12 +42,15 @@ constexpr int kDefaultMinTiles = 1;  // round CTAs kept: one per tile of the rou
 constexpr int64_t kWlSlack = 1 << 19;  // worklist slots beyond `edges` (scan chunk tails)
 constexpr int kLearnedMinEdges = 1 << 20;
 // Single graphs up to this many entries are solved in one launch (k_group):
-// RMAT-14 156 us against 200 with a launch per pass, ER 200k 295 against 327,
-// the 1000 x 1000 grid (4.0M entries) 456 against 481.
+// RMAT-14 156 us against 200 with a launch per pass, ER 200k 295 against 327.
+// At 4.0M entries ER 500k takes 338 against 360 and RMAT-16 207 against 219, but
+// a grid 437 against 416; at 4.5M 367 against 388, 219 against 221 and 463
+// against 437; at 8.0M ER 1M 505 against 491, a geometric graph 479 against 461
+// and a grid 663 against 625.
 constexpr int kGroupEdges = 1 << 22;
-// and of up to this many entries by one cluster (k_cluster), alone on one CTA
-// up to kClusterShare
-constexpr int kClusterEdges = 1 << 16;
+// and of up to this many entries and vertices by one cluster (k_cluster), alone
+// on one CTA up to kClusterShare entries
+constexpr int kClusterEdges = 1 << 16, kClusterNodes = 1 << 15;
 constexpr int kClusterShare = 1 << 14;
 }  // namespace
 
@@ -542,14 +545,19 @@ int prepare_cluster_kernels() {
 
 // CTAs of the cluster that solves a graph alone (k_cluster), 0 = k_group does.
 // One CTA up to kClusterShare entries and what its shared memory holds, else
-// one per half of that. Measured against k_group: ER of 1000 vertices 57 us
-// (one CTA) against 99, ER 4000 107 (4 CTAs) against 156, 16 000-vertex grid
-// (8 CTAs) 138 against 165; from 128K entries on k_group is the faster one.
+// one per quarter of that, in entries or vertices: the roots pass looks at every
+// vertex, and a thread's unions and walks follow one another (the path of 16 000
+// equal weights 55 us on 8 CTAs, 85 on 4; ER 3000 98 against 108). Measured
+// against k_group: ER of 1000 vertices 57 us (one CTA) against 99, ER 4000 107
+// (4 CTAs) against 156, 16 000-vertex grid (8 CTAs) 138 against 165; from 128K
+// entries on k_group is the faster one, and beyond kClusterNodes vertices with
+// few entries too (0.2 per vertex: 40 000 57 us against 82, 60 000 64 against
+// 122; 32 000 84 against 59 on 8 CTAs).
 int cluster_ctas(int n, int m, unsigned wl_cap) {
-  if (m > kClusterEdges || n > kClusterEdges || (unsigned)m > wl_cap) return 0;
+  if (m > kClusterEdges || n > kClusterNodes || (unsigned)m > wl_cap) return 0;
   if (m <= kClusterShare && n <= kClVertices) return 1;
   int c = 2;
-  while (c < kClMaxCtas && m > c * (kClusterShare / 2)) c *= 2;
+  while (c < kClMaxCtas && std::max(m, n) > c * (kClusterShare / 4)) c *= 2;
   return c;
 }
 
