@@ -290,8 +290,9 @@ typedef struct ecl_mst_stats {
   float ms_rounds;         /* device time of the round kernels                  */
   float ms_scan;           /* device time of everything else (scans, prep,
                               features, flatten)                                */
-  /* breakdown (microseconds); us_scan from CUDA events, us_round from the
-   * device clock at the round kernel's barriers:                            */
+  /* breakdown (microseconds); us_scan from CUDA events (from the device clock
+   * where one launch does the whole solve, whose launch cost then counts in
+   * ms_scan), us_round from the device clock at the rounds' barriers:        */
   float us_scan[2][3];     /* [0]: {features + prep + light scan, features +
                               prep, light scan kernel}; [1]: {flatten + heavy
                               scan, flatten (and the rounds of the heavy list

@@ -348,6 +348,10 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
   if (tid < 3) sm.total[tid] = 0;
   if (tid == 0) sm.cursor = 0;
   sy.sync();
+  auto step_done = [&](int step) {
+    if (rank == 0 && tid == 0) st->t_step[step] = globaltimer_ns();
+  };
+  step_done(kStepStart);
   if (rank == 0 && g.batch && g.mode == ECL_THRESH_QUANTILE && g.quantile < 1.0f) {
     if (tid == 0) batch_quantile(st, g.eweight, m, g.quantile);
   } else if (rank == 0) {
@@ -380,9 +384,11 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
   int4* l0 = g.wl0 + region;
   int4* l1 = g.wl1 + region;
   unsigned pass_no = 0;
+  step_done(kStepPrep);
   cl_scan<kLight>(g, M, ctas, thr, l0, sm);
   __syncthreads();
   cl_rounds(g, M, sy, 0, -1, l0, l1, pass_no, sm);
+  step_done(kStepLight);
   if (!filtered) return;
   __syncthreads();
   if (tid == 0) sm.cursor = 0;
@@ -401,9 +407,11 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
   }
   sy.sync();
   const int giant = (int)ld_volatile((const unsigned*)&st->giant);
+  step_done(kStepFlatten);
   cl_scan<kHeavy>(g, M, ctas, thr, l0, sm);
   __syncthreads();
   cl_rounds(g, M, sy, 1, giant, l0, l1, pass_no, sm);
+  step_done(kStepHeavy);
 }
 
 template <bool kOne>

@@ -674,12 +674,9 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
     ca.parent = sl.parent;
     ca.minv = sl.minv0;
     ca.st = c->st;
-    if (timed)  // one launch: all of it counts as rounds
-      for (int k : {5, 1}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
     const int r = enqueue_cluster(ca, ctas, o, s);
     if (r) return r;
-    if (timed)
-      for (int k : {2, 6, 3, 4}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[4], s));
     return ECL_OK;
   }
   if (m <= kGroupEdges && one_launch) {
@@ -698,13 +695,10 @@ int enqueue_solve(ecl_mst_ctx* c, const ecl_graph* g, unsigned char* d_inMST, co
     ga.wl1 = c->wl[1];
     ga.wl_cap = c->wl_cap;
     ga.st = c->st;
-    if (timed)  // one launch: all of it counts as rounds
-      for (int k : {5, 1}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
     const int r = enqueue_group(ga, o, c->wl_cap - (unsigned)(c->wl_full ? m : m / 2), c->sm_count, c->group_grid, s,
                                 win_all);
     if (r) return r;
-    if (timed)
-      for (int k : {2, 6, 3, 4}) ECL_CUDA_TRY(cudaEventRecord(c->ev[k], s));
+    if (timed) ECL_CUDA_TRY(cudaEventRecord(c->ev[4], s));
     return ECL_OK;
   }
   PrepArgs pa{};
@@ -870,6 +864,18 @@ int fill_stats(ecl_mst_ctx* c, ecl_mst_stats* stats, bool timed, bool breakdown 
   }
   if (timed && !breakdown) {  // a replayed graph: only the whole solve is timed
     cudaEventElapsedTime(&stats->ms_total, c->ev[0], c->ev[4]);
+  } else if (timed && h.t_step[kStepStart]) {  // one launch: the kernel's own times
+    cudaEventElapsedTime(&stats->ms_total, c->ev[0], c->ev[4]);
+    auto us = [](u64 from, u64 to) { return from && to > from ? (float)(to - from) * 1e-3f : 0.f; };
+    const u64 *t = h.t_step, *r = h.t_round_start;
+    float(*sc)[3] = stats->us_scan;
+    sc[0][1] = us(t[kStepStart], t[kStepPrep]);
+    sc[0][2] = us(t[kStepPrep], r[0]);
+    sc[1][1] = us(t[kStepLight], t[kStepFlatten]);
+    sc[1][2] = us(t[kStepFlatten], r[1]);
+    for (int p = 0; p < 2; p++) sc[p][0] = sc[p][1] + sc[p][2];
+    stats->ms_rounds = (us(r[0], t[kStepLight]) + us(r[1], t[kStepHeavy])) * 1e-3f;
+    stats->ms_scan = std::max(0.f, stats->ms_total - stats->ms_rounds);
   } else if (timed) {
     float t01, t12, t23, t34, t04;
     cudaEventElapsedTime(&t01, c->ev[0], c->ev[1]);

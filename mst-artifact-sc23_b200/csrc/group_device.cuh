@@ -216,6 +216,10 @@ __device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
   const unsigned gid = rank * kGroupThreads + tid, stride = ctas * kGroupThreads;
   const int n = g.nodes, m = g.edges;
   if (m == 0) return true;
+  auto step_done = [&](int step) {
+    if (rank == 0 && tid == 0) st->t_step[step] = globaltimer_ns();
+  };
+  step_done(kStepStart);
   if (rank == 0) {
     PrepArgs pa{};
     pa.nodes = n;
@@ -239,10 +243,12 @@ __device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
   if (bad) atomicOr(&st->error, kErrFormat);
   if (!sy.sync()) return false;
   if (ld_volatile(&st->error) & kErrFormat) return true;  // only set before the barrier: the whole group
+  step_done(kStepPrep);
   group_scan<kLight>(g, rank, ctas, sm);
   if (!sy.sync()) return false;
   const int filtered = st->filtered;
   if (!group_rounds(g, 0, -1, sy, sm)) return false;
+  step_done(kStepLight);
   if (!filtered) return true;
   // parent[v] = root(v), and the tree most entries point into (a vote of 32)
   for (unsigned v = gid; v < (unsigned)n; v += stride) {
@@ -260,9 +266,12 @@ __device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
   }
   if (!sy.sync()) return false;
   const int giant = (int)ld_volatile((const unsigned*)&st->giant);
+  step_done(kStepFlatten);
   group_scan<kHeavy>(g, rank, ctas, sm);
   if (!sy.sync()) return false;
-  return group_rounds(g, 1, giant, sy, sm);
+  if (!group_rounds(g, 1, giant, sy, sm)) return false;
+  step_done(kStepHeavy);
+  return true;
 }
 
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) k_group(GroupArgs g) {

@@ -126,6 +126,11 @@ struct ListCount {
   unsigned slots, kept;  // slots reserved (null padding included), entries
 };
 
+// Times (globaltimer) of a solve in one launch, which has no events between its
+// steps: its start, and the ends of prep, the light phase's rounds, flatten and
+// the heavy phase's rounds (the scans end where t_round_start is).
+enum : int { kStepStart = 0, kStepPrep, kStepLight, kStepFlatten, kStepHeavy, kSteps };
+
 // Control block of one solve, zeroed before every solve.
 struct alignas(128) DevState {
   int threshold;       // light phase keeps w <= threshold
@@ -143,6 +148,7 @@ struct alignas(128) DevState {
   // [phase][2r] after round r's find/min pass, [phase][2r+1] after its mark pass
   u64 t_round_start[2];
   u64 t_round[2][2 * ECL_MAX_ROUNDS];
+  u64 t_step[kSteps];  // solves in one launch: ends of their steps (kStepStart ...)
   ListCount lists[4];
   unsigned split_light;  // light entries up to this weight (as unsigned) go to list light 0
   unsigned split_heavy;  // heavy entries up to this weight go to list mid, if
