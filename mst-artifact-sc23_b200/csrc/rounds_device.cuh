@@ -621,6 +621,9 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, Sync& 
         const bool valid[2] = {tid == 0, false};
         bor_roots_step<2>(a, v, valid, false, b.skip, rout, rctr, flip, s);
       }
+      // Every warp has read the CTA's count of entries before it is cleared: the
+      // steps' CTA barriers see to that, but steps without a list have none.
+      __syncthreads();
     } else {
       const unsigned cnt = all ? (unsigned)a.nodes : b.C;
       for (unsigned base = start * T * U; base < cnt; base += stride * T * U, flip ^= 1) {
@@ -636,9 +639,6 @@ __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, Sync& 
       }
     }
     if (stamp) st->root_cnt[a.list][(b.flips + 1) % 3] = 0;  // the next roots pass's counter
-    // Every warp has read its count of the CTA's entries before it is cleared:
-    // the steps' CTA barriers see to that, but steps without a list have none.
-    if (b.first && !all && !rout) __syncthreads();
     if (tid == 0) s.cursor = 0;
     if (!sy.sync()) break;
     if (stamp) st->t_round[ph][2 * b.r - 1] = globaltimer_ns();
