@@ -427,12 +427,11 @@ int ecl_mst_run_batch_device(ecl_batch_ctx* ctx, const ecl_batch* batch,
                              uint8_t* d_inMST, const mst_opts* opts, void* stream,
                              ecl_batch_stats* stats);
 
-/* Autotuner: times candidate schedules (small-graph cutoff, degree split
- * and, when *base asks for the learned schedule, learned against the
- * reference heuristic for the large graphs; then, unless *base sets them,
- * the large graphs' streams and round-kernel CTAs per SM, and the cutoff
- * again with those) on the batch and
- * writes the fastest into *best (a copy of *base with those fields set).
+/* Autotuner: times candidate schedules (small-graph cutoff and, when *base
+ * asks for the learned schedule, learned against the reference heuristic for
+ * the large graphs; then, unless *base sets them, the large graphs' streams
+ * and round-kernel CTAs per SM, and the cutoff again with those) on the batch
+ * and writes the fastest into *best (a copy of *base with those fields set).
  * The answer is the same for every candidate; only the time differs. */
 int ecl_batch_autotune(ecl_batch_ctx* ctx, const ecl_batch* batch, uint8_t* d_inMST,
                        const mst_opts* base, mst_opts* best, float* best_ms);
@@ -454,7 +453,8 @@ void ecl_free_device_batch(ecl_batch* b);
 /* A 16 -> 64 -> 64 -> 2 ReLU MLP (fp32) maps 16 graph features to the light-
  * phase filter quantile (output 0: log2 q minus the log2 of the reference
  * heuristic's quantile, (idx+1)/21 or 1 when it does not filter; a total
- * >= 0 means no filter) and the scans' degree split (output 1, log2 split). It changes the schedule only.
+ * >= 0 means no filter) and a degree split (output 1, log2 split, which is
+ * only reported). It changes the schedule only.
  * Parameter blob (ECL_MLP_PARAMS floats): W1[16][64], b1[64], W2[64][64],
  * b2[64], W3[64][2], b3[2], feature mean[16], feature std[16]. */
 #define ECL_MLP_INPUTS 16

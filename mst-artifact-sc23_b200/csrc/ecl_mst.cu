@@ -2070,21 +2070,18 @@ extern "C" int ecl_batch_autotune(ecl_batch_ctx* c, const ecl_batch* b, uint8_t*
   };
   int st;
   const int cutoffs[] = {c->cap / 8, c->cap / 4, c->cap / 2, c->cap};
-  // 1. small-graph cutoff, degree split and schedule. The learned
-  //    schedule (large graphs only) is kept only where it beats the
-  //    reference heuristic on this batch.
+  // 1. small-graph cutoff and schedule. The learned schedule (large graphs
+  //    only) is kept only where it beats the reference heuristic on this
+  //    batch. (degree_split changes no kernel's work and stays as in *base.)
   const int modes[] = {o0.threshold_mode, ECL_THRESH_HEURISTIC};
   const int nmodes = o0.threshold_mode == ECL_THRESH_LEARNED ? 2 : 1;
   for (int mi = 0; mi < nmodes; mi++)
     for (int cut : cutoffs) {
       if (cut < 1) continue;
-      for (int sp : {8, 16}) {
-        mst_opts o = o0;
-        o.threshold_mode = modes[mi];
-        o.batch_small_edges = cut;
-        o.degree_split = sp;
-        if ((st = trial(o))) return st;
-      }
+      mst_opts o = o0;
+      o.threshold_mode = modes[mi];
+      o.batch_small_edges = cut;
+      if ((st = trial(o))) return st;
     }
   // 2. the large graphs' streams and round CTAs per SM, unless *base sets them
   if (best_o.batch_large_streams == 0 && best_o.ctas_per_sm == 0) {

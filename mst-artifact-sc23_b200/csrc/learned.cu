@@ -2,8 +2,8 @@
 // and a small MLP (16 -> 64 -> 64 -> 2, ReLU, fp32) with hand-written CUDA
 // inference, gradient and training (Adam) kernels. The network maps the
 // features to the light-phase filter quantile (output 0, as log2 q relative
-// to the reference heuristic's quantile) and the scan's degree split
-// (output 1, as log2 split). Only the schedule changes;
+// to the reference heuristic's quantile) and a degree split (output 1, as log2
+// split, which is only reported). Only the schedule changes;
 // the forest is unique under the (weight, index) order, so the answer does
 // not (for non-negative weights). The reference heuristic (ECL_MST.cu:432-440)
 // remains the fallback when no weights are loaded.
@@ -237,8 +237,7 @@ __global__ void k_mlp_apply(const float* pg, const FeatAcc* acc, const int* sort
   st->quantile = r.quantile;
   st->filtered = r.filtered;
   st->threshold = r.threshold;
-  st->learned_split = r.split;
-  st->split = r.split;  // read by the scans (k_prep leaves it alone in this mode)
+  st->split = r.split;  // reported (k_prep leaves it alone in this mode)
   // the lists' split weights, from the same sorted sample (read as unsigned:
   // negative weights come after the others)
   st->split_light = 0xffffffffu;

@@ -135,13 +135,12 @@ enum : int { kStepStart = 0, kStepPrep, kStepLight, kStepFlatten, kStepHeavy, kS
 struct alignas(128) DevState {
   int threshold;       // light phase keeps w <= threshold
   int filtered;        // 1 = light + heavy phase, 0 = one unfiltered phase
-  int split;           // degree split between the thread and the chunk tier
+  int split;           // degree split asked for or learned (only reported: the scans need none)
   unsigned error;      // kErr* bits
   unsigned bar_count;  // grid barrier: CTAs arrived in the current generation
   unsigned bar_gen;    // grid barrier: generation counter
   int rounds[2];       // Boruvka rounds per phase
   float quantile;      // learned / quantile modes: filter quantile in [0,1]
-  int learned_split;   // learned mode: predicted degree split
   u64 atomics;         // guarded atomicMin issued (stats mode)
   unsigned wl_count[2][ECL_MAX_ROUNDS + 1];  // [phase][r] = entries entering round r
   // globaltimer stamps taken by CTA 0 at phase boundaries (diagnostics):
