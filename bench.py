@@ -579,13 +579,17 @@ def main():
     # Ablation (the reference's deoptimization pipeline, generate_deoptimize_tables.py:6-14,
     # restated for this engine): the reference heuristic schedule with techniques switched off,
     # cumulatively for the reference's NoAtomicGuards / NoWarp / NoFilter steps, and one at a
-    # time for this engine's own techniques. Every variant must give the same inMST.
+    # time for this engine's own techniques. The switches vary a round kernel of their own, so
+    # they are compared with that kernel unvaried ("variant_base"); "base" is the default solve.
+    # Every variant must give the same inMST.
     ablation = None
     if not args.profile and not args.no_ablation:
         E_ = E
         nag_nw = E_.FLAG_NO_GUARDS | E_.FLAG_NO_WARP_COOP
         nipc = nag_nw | E_.FLAG_NO_IMPLICIT_COMPRESSION
         series = [("base", 0, E_.THRESH_HEURISTIC),
+                  ("no_small_tail", E_.FLAG_NO_SMALL_TAIL, E_.THRESH_HEURISTIC),
+                  ("variant_base", E_.FLAG_VARIANT_BASE, E_.THRESH_HEURISTIC),
                   ("NAG", E_.FLAG_NO_GUARDS, E_.THRESH_HEURISTIC),
                   ("NAG_NW", nag_nw, E_.THRESH_HEURISTIC),
                   ("NAG_NW_NF", nag_nw, E_.THRESH_NONE),
@@ -596,9 +600,8 @@ def main():
                   ("NAG_NW_NF_NIPC_NT_NDD_NEB", nipc | E_.FLAG_NO_TUPLES | E_.FLAG_NO_DATA_DRIVEN
                    | E_.FLAG_NO_EDGE_BASED, E_.THRESH_NONE),
                   ("with_dedup", E_.FLAG_DEDUP, E_.THRESH_HEURISTIC),
-                  ("no_find_cache", E_.FLAG_NO_FIND_CACHE, E_.THRESH_HEURISTIC),
-                  ("no_small_tail", E_.FLAG_NO_SMALL_TAIL, E_.THRESH_HEURISTIC)]
-        ablation, base_ms, ref_hash = {}, None, None
+                  ("no_find_cache", E_.FLAG_NO_FIND_CACHE, E_.THRESH_HEURISTIC)]
+        ablation, ref_hash, against = {}, None, "base"
         for name, flags, tmode in series:
             o = E_.make_opts(mode=tmode, degree_split=args.split, flags=flags)
             ms = []
@@ -612,9 +615,11 @@ def main():
             h = hash(d_out[: g.edges].cpu().numpy().tobytes())
             ref_hash = h if ref_hash is None else ref_hash
             m = float(np.mean(ms))
-            base_ms = m if base_ms is None else base_ms
-            ablation[name] = {"ms": m, "gedges_s": g.edges / (m * 1e-3) / 1e9, "slowdown": m / base_ms,
+            ablation[name] = {"ms": m, "gedges_s": g.edges / (m * 1e-3) / 1e9, "against": against,
+                              "slowdown": m / ablation[against]["ms"] if against in ablation else 1.0,
                               "inMST_identical": h == ref_hash}
+            if name == "variant_base":
+                against = name
 
     # one extra solve counting the guarded atomics for the byte model
     st_atom = ctx.run_device(g.nodes, g.edges, d_ni.data_ptr(), d_nl.data_ptr(), d_ew.data_ptr(),

@@ -192,8 +192,12 @@ enum {
                                    set-aside takes L2 from the heavy scan)      */
   ECL_FLAG_STATS = 1 << 1,      /* count guarded atomics (slower; off in timing) */
   ECL_FLAG_NO_SMALL_TAIL = 1 << 2, /* keep every round grid-wide (ablation)     */
-  /* Ablation switches: each turns one technique of the round kernel off, to
-   * measure what it buys (the answer is unchanged). NO_GUARDS is the
+  /* Ablation switches: each turns one technique of a round kernel off, to
+   * measure what it buys (the answer is unchanged). That kernel is not the
+   * default one: VARIANT_BASE runs it with every technique on, and is what
+   * the switches are to be compared with (NO_SMALL_TAIL alone varies the
+   * default kernel). In a batch they apply to the graphs that the grid-wide
+   * engines solve. NO_GUARDS is the
    * reference's NoAtomicGuards variant (Deoptimizations/
    * ECL_MST_NoAtomicGuards.cu:222-223); NO_WARP_COOP stands for its NoWarp
    * variant, applied to this engine's warp/CTA cooperation on shared reps. */
@@ -228,9 +232,11 @@ enum {
                                       phase's whole list, nothing is compacted
                                       (..._NoDataDriven.cu:166-180, 263-270;
                                       implies NO_IMPLICIT_COMPRESSION)         */
-  ECL_FLAG_NO_EDGE_BASED = 1 << 11 /* vertex-centric rounds over the CSR, one
+  ECL_FLAG_NO_EDGE_BASED = 1 << 11, /* vertex-centric rounds over the CSR, one
                                       thread per vertex, no worklists
                                       (..._NoEdgeBased.cu:152-195)             */
+  ECL_FLAG_VARIANT_BASE = 1 << 12  /* the ablation switches' round kernel with
+                                      none of its techniques off               */
 };
 
 typedef struct mst_opts {

@@ -253,7 +253,8 @@ unsigned round_ablation(int flags) {
   return ((flags & ECL_FLAG_NO_GUARDS) ? kAblNoGuards : 0u) | ((flags & ECL_FLAG_NO_WARP_COOP) ? kAblNoCoop : 0u) |
          ((flags & ECL_FLAG_DEDUP) ? kDedup : 0u) | ((flags & ECL_FLAG_NO_FIND_CACHE) ? kAblNoFindCache : 0u) |
          ((flags & ECL_FLAG_NO_IMPLICIT_COMPRESSION) ? kAblNoIPC : 0u) |
-         ((flags & ECL_FLAG_NO_TUPLES) ? kAblNoTuples : 0u) | ((flags & ECL_FLAG_NO_DATA_DRIVEN) ? kAblNoDD : 0u);
+         ((flags & ECL_FLAG_NO_TUPLES) ? kAblNoTuples : 0u) | ((flags & ECL_FLAG_NO_DATA_DRIVEN) ? kAblNoDD : 0u) |
+         ((flags & ECL_FLAG_VARIANT_BASE) ? kAblBase : 0u);
 }
 
 // The reference's later ablation steps, which only the single-graph engine runs.

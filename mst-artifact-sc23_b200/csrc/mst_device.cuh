@@ -145,6 +145,7 @@ enum : unsigned {
   kAblNoDD = 64u,      // NoDataDriven: every round reads the phase's whole list
                        // and nothing is compacted; the rounds end when no entry
                        // joins two trees (..._NoDataDriven.cu:166-180, 263-270)
+  kAblBase = 128u,     // nothing off: what the others are compared with
 };
 // Switches under which worklist entries keep their endpoints (no rewrite to reps)
 constexpr unsigned kAblKeepEnds = kAblNoIPC | kAblNoTuples | kAblNoDD;
