@@ -1495,8 +1495,10 @@ constexpr int kDefaultLargeStreams = 4;  // measured: 957 large graphs of the mi
 
 }  // namespace
 
-// Size classes of a batch's small graphs (batch_small).
-constexpr int kBatchClasses = 4;
+// Size classes of a batch's small graphs (batch_small) and the CTAs of their
+// clusters. The last one keeps parent[] and the slots in shared memory.
+constexpr int kBatchClasses = 5;
+constexpr int kClassCtas[kBatchClasses] = {8, 4, 2, 1, 1};
 
 struct ecl_batch_ctx {
   int device = 0;
@@ -1506,8 +1508,9 @@ struct ecl_batch_ctx {
   int64_t max_nodes = 0, max_edges = 0;
   int cap = 0;        // per-CTA scratch: vertices and CSR entries
   // scratch for small_grid graphs of `cap` vertices and entries; a run divides
-  // it among the clusters of its size classes (at most sm_count / size each)
-  int small_grid = 0;
+  // it among the clusters of its size classes (at most sm_count / size each,
+  // state_count in all)
+  int small_grid = 0, state_count = 0;
   int* parent_pool = nullptr;
   u64* minv_pool = nullptr;
   int4* wl_pool = nullptr;
@@ -1601,12 +1604,13 @@ extern "C" int ecl_batch_ctx_create(int device, int32_t max_graphs, int64_t max_
     return fail(st);
   if ((st = cuda_status(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)))) return fail(st);
   c->small_grid = 2 * c->sm_count;
+  for (int size : kClassCtas) c->state_count += std::max(1, c->sm_count / size);
   if ((st = prepare_cluster_kernels())) return fail(st);
   const size_t ctas = (size_t)c->small_grid, cap = (size_t)c->cap;
   if ((st = cuda_status(cudaMalloc(&c->parent_pool, ctas * cap * sizeof(int))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->minv_pool, ctas * cap * sizeof(u64))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->wl_pool, ctas * 2 * cap * sizeof(int4))))) return fail(st);
-  if ((st = cuda_status(cudaMalloc(&c->states, ctas * sizeof(DevState))))) return fail(st);
+  if ((st = cuda_status(cudaMalloc(&c->states, (size_t)c->state_count * sizeof(DevState))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->d_graphs, (size_t)max_graphs * sizeof(GraphDesc))))) return fail(st);
   if ((st = cuda_status(cudaMalloc(&c->d_queue, kBatchClasses * sizeof(unsigned))))) return fail(st);
   for (auto& q : c->cls_stream)
@@ -1639,21 +1643,29 @@ namespace {
 
 // The graphs solved by clusters. A graph's cluster has two CTAs or more if one
 // cannot hold its vertices (kClVertices), and as many as its share of the
-// batch's entries asks for, so that no graph is worked on much longer than an
-// even split of the batch over the chip takes (twice that share, rounded up to
-// 1, 2, 4 or 8): a batch of thousands runs one CTA to a graph, a few graphs run
-// on as much of the chip as they can use. Largest first within a class; the
-// classes run side by side, the largest clusters launched first. 398 graphs of
-// 1000 to 60 000 vertices: 1.9 ms against 7.1 with one CTA to every graph.
+// batch's work asks for (entries, or vertices where these are more), so that no
+// graph is worked on much longer than an even split of the batch over the chip
+// takes (twice that share, rounded up to 1, 2, 4 or 8): a batch of thousands
+// runs one CTA to a graph, a few graphs run on as much of the chip as they can
+// use. Sparse graphs that one CTA cannot hold run on one all the same: latency
+// is what they cost, and twice as many side by side hide it (400 of 17 000
+// vertices and 1000 edges 0.12 ms against 0.25 on two CTAs each; for graphs of
+// more entries than vertices the rule loses where a batch has few of them, 398 of
+// 1000 to 60 000 vertices 2.16 ms against 2.11). Largest first within a class; the
+// classes run side by side, the largest clusters launched first. Those 398
+// graphs took 7.1 ms with one CTA to every graph.
 int batch_small(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& small, uint8_t* d_inMST,
                 const mst_opts* o, cudaStream_t s) {
   const int S = (int)small.size();
+  auto fits = [&](int g) { return b->nodes[g] <= kClVertices; };
+  auto work = [&](int g) { return (int64_t)(fits(g) ? b->edges[g] : std::max(b->edges[g], b->nodes[g])); };
   int64_t total = 0;
-  for (int g : small) total += b->edges[g];
+  for (int g : small) total += work(g);
   const int64_t share = std::max<int64_t>(kClTile, total / (2 * c->sm_count));
-  auto class_of = [&](int g) {  // class k: 8 >> k CTAs
-    int k = b->nodes[g] > kClVertices ? kBatchClasses - 2 : kBatchClasses - 1;
-    while (k > 0 && b->edges[g] > (8 >> k) * share) k--;
+  auto class_of = [&](int g) {
+    if (fits(g) && work(g) <= share) return kBatchClasses - 1;
+    int k = !fits(g) && b->edges[g] < b->nodes[g] ? 3 : 2;
+    while (k > 0 && work(g) > kClassCtas[k] * share) k--;
     return k;
   };
   std::vector<int> order(small);
@@ -1681,22 +1693,26 @@ int batch_small(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& sm
   ba.explicit_thr = o->threshold;
   ba.quantile = o->quantile;
   ba.count_atomics = (o->flags & ECL_FLAG_STATS) ? 1 : 0;
+  // clusters of every class and the graph size their scratch is for; all of a
+  // class at once if the pool has room, else its part of the pool
+  int64_t cap[kBatchClasses], want[kBatchClasses], needed = 0, least = 0;
+  for (int k = 0; k < kBatchClasses; k++) {
+    cap[k] = 0;
+    for (int i = first[k]; i < first[k + 1]; i++) cap[k] = std::max<int64_t>(cap[k], std::max(descs[i].nodes, descs[i].edges));
+    cap[k] = (cap[k] + 3) & ~(int64_t)3;
+    want[k] = std::min(first[k + 1] - first[k], std::max(1, c->sm_count / kClassCtas[k]));
+    needed += want[k] * cap[k];
+    least += cap[k];
+  }
   const int64_t pool = (int64_t)c->small_grid * c->cap;
   int64_t used = 0;  // pool entries given out
   int states = 0, forked = 0;
   ECL_CUDA_TRY(cudaEventRecord(c->cls_fork, s));
   for (int k = 0; k < kBatchClasses; k++) {
-    const int count = first[k + 1] - first[k], size = 8 >> k;
+    const int count = first[k + 1] - first[k], size = kClassCtas[k];
     if (count <= 0) continue;
-    int64_t cap = 1;
-    for (int i = first[k]; i < first[k + 1]; i++)
-      cap = std::max<int64_t>(cap, std::max(descs[i].nodes, descs[i].edges));
-    cap = (cap + 3) & ~(int64_t)3;
-    // the classes after this one keep at least one cluster's worth of the pool
-    const int later = kBatchClasses - 1 - k;
-    const int64_t fit = (pool - later * ((int64_t)c->cap + 3) - used) / cap;
-    const int clusters = (int)std::min<int64_t>({(int64_t)count, (int64_t)std::max(1, c->sm_count / size), fit,
-                                                 (int64_t)c->small_grid - later - states});
+    // (more than the pool: the parts add up to pool - least, one cluster each to least)
+    const int clusters = (int)(needed <= pool ? want[k] : std::max<int64_t>(1, want[k] * (pool - least) / needed));
     ba.graphs = c->d_graphs + first[k];
     ba.count = count;
     ba.queue = c->d_queue + k;
@@ -1704,15 +1720,15 @@ int batch_small(ecl_batch_ctx* c, const ecl_batch* b, const std::vector<int>& sm
     ba.parent_pool = c->parent_pool + used;
     ba.minv_pool = c->minv_pool + used;
     ba.wl_pool = c->wl_pool + 2 * used;
-    ba.cap = cap;
-    used += clusters * cap;
+    ba.cap = cap[k];
+    used += clusters * cap[k];
     states += clusters;
     cudaStream_t q = s;
     if (first[k + 1] < S) {  // the last class runs on the caller's stream
       q = c->cls_stream[forked];
       ECL_CUDA_TRY(cudaStreamWaitEvent(q, c->cls_fork, 0));
     }
-    const int st = size == 1 ? launch_cluster(k_batch_cluster<true>, 1, clusters, kClThreads, kClSmem, q, ba)
+    const int st = k == kBatchClasses - 1 ? launch_cluster(k_batch_cluster<true>, 1, clusters, kClThreads, kClSmem, q, ba)
                              : launch_cluster(k_batch_cluster<false>, size, clusters, kClThreads, 0, q, ba);
     if (st) return st;
     if (q != s) ECL_CUDA_TRY(cudaEventRecord(c->cls_join[forked++], q));
