@@ -5,11 +5,10 @@
    degree 8, 16 or 32), RMAT (.57, .19, .19; edge factor 8, 16 or 32) and
    random geometric 2D (average degree 3), vertex counts log-uniform in
    [--nmin, --nmax], weights uniform in [1, W] with W one of 2^20, 2^24, 2^30.
-2. Label sweep: solve every graph with each of 16 filter quantiles x the 3
-   degree splits (repeats: the scans work by entries and do not depend on
-   it) and keep the device times (best of
-   --reps timed runs after one warm-up; repeated solves replay their captured
-   CUDA graph). Every setting gives the same forest.
+2. Label sweep: solve every graph with each of 16 filter quantiles and keep
+   the device times (best of --reps timed runs after one warm-up; repeated
+   solves replay their captured CUDA graph). Every setting gives the same
+   forest.
 3. Label each graph with a soft minimum over the sweep (log2 quantile
    relative to the reference heuristic's, log2 split) and train the
    16 -> 64 -> 64 -> 2 MLP with the library's CUDA training kernel (Adam, one
@@ -42,7 +41,9 @@ sys.path.insert(0, HERE)
 import ecl_mst as E  # noqa: E402
 
 QUANTILES = [0.005, 0.01, 0.02, 0.03, 0.05, 0.07, 0.1, 0.15, 0.2, 0.3, 0.4, 0.5, 0.65, 0.8, 0.9, 1.0]
-SPLITS = [4, 8, 16]  # degree splits (the scans no longer depend on them: repeats, best time kept)
+# Degree splits, the sweep tables' second axis: no kernel's work depends on the split any more, so a
+# quantile is solved once and its time stands for all of them
+SPLITS = [4, 8, 16]
 FAMILIES = ["grid", "er", "rmat", "rgg"]
 TRAIN_SEED0, HELDOUT_SEED0 = 200_000, 900_000
 
@@ -86,9 +87,7 @@ def sweep(ctx, dg, out, reps):
     feat = E.graph_features(dg.nodes, dg.edges, dg.d_nindex, dg.d_nlist, dg.d_eweight)
     times = np.zeros((len(QUANTILES), len(SPLITS)), np.float32)
     for qi, q in enumerate(QUANTILES):
-        for si, sp in enumerate(SPLITS):
-            times[qi, si] = solve_ms(ctx, dg, out, E.make_opts(mode=E.THRESH_QUANTILE, quantile=q, degree_split=sp),
-                                     reps)
+        times[qi] = solve_ms(ctx, dg, out, E.make_opts(mode=E.THRESH_QUANTILE, quantile=q), reps)
     heur = solve_ms(ctx, dg, out, E.make_opts(), reps)
     return feat, times, heur
 
@@ -124,7 +123,7 @@ def predicted_setting(pr, n, m):
     q = 1.0 if lq >= NO_FILTER_LOG2Q else 2.0 ** lq
     sp = int(round(min(max(float(pr[1]), 1.0), 6.0)))
     qi = int(np.argmin([abs(np.log2(a) - np.log2(q)) for a in QUANTILES]))
-    si = 0 if sp <= 2 else (1 if sp == 3 else 2)  # E = 4 for splits <= 4, 8 for 8, 16 above
+    si = 0 if sp <= 2 else (1 if sp == 3 else 2)  # the split nearest on the tables' axis
     return qi, si
 
 
