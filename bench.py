@@ -141,7 +141,8 @@ class ClockSampler:
 
 
 def round_kernel_bytes(st, nodes, entry_bytes=16, atomics=None):
-    """Algorithmic bytes of the round kernels of one solve.
+    """Algorithmic bytes of the round kernels of one solve by the ablation switches'
+    round kernel (k_rounds; round_pass_bytes has the default kernels').
 
     Per round with W_in real entries in and W_out kept (both phases):
       first round of a phase (in place on the scan's list, no find, no copy):
@@ -174,12 +175,84 @@ def round_kernel_bytes(st, nodes, entry_bytes=16, atomics=None):
 
 
 def scan_kernel_bytes(st, nodes, edges, entry_bytes=16):
-    """Light scan: nindex + nlist + eweight + init of parent/min slots + appended entries.
+    """Scans that read both entry arrays whole (scan_pass_bytes has the default kernels').
+    Light scan: nindex + nlist + eweight + init of parent/min slots + appended entries.
     Heavy scan: flatten (parent read+write) + nindex + nlist + eweight + appended."""
     b = 4 * (nodes + 1) + 8 * edges + 20 * nodes + entry_bytes * st["scan_kept"][0]
     if st["filtered"]:
         b += 8 * nodes + 4 * (nodes + 1) + 8 * edges + entry_bytes * st["scan_kept"][1]
     return b
+
+
+def list_starts(w, rounds):
+    """The rounds of a phase at which a list begins (its entries by round only shrink)."""
+    return [r for r in range(rounds) if r == 0 or w[r] > w[r - 1]]
+
+
+def round_pass_bytes(st, atomics):
+    """Bytes that the rounds' three passes cannot do without, both phases, for
+    `atomics` guarded atomics issued. Per round with W real entries in and K kept:
+      offer   16 W (read), 8 K per end offered to (guard reads) and, but for the
+              first round of a phase's main list (roots already, kept in place,
+              K = W), 2 * 4 W (parent) and 16 K (compacted write)
+      mark    16 K (read), 8 K per end offered to (slot reads)
+    Both ends of an entry are offered to, but in all lists after the first one
+    the largest tree, at one end of nearly every entry, is not: one end counts.
+    16 per atomicMin. The roots pass (24 per live root) is left out: the
+    statistics do not say how many there are.
+    """
+    total = 16 * atomics
+    for p in range(2):
+        w, rounds = st["wl_real"][p], st["rounds"][p]
+        starts = list_starts(w, rounds)
+        for s, e in zip(starts, starts[1:] + [rounds]):
+            # the light phase's first list and the heavy list; mid and light 1 hold no roots
+            in_place = s == (0 if p == 0 else starts[-1])
+            ends = 2 if p == 0 and s == 0 else 1
+            for r in range(s, e):
+                win, wout = w[r], w[r + 1] if r + 1 < e else 0
+                total += 16 * win + 8 * ends * wout
+                if not (in_place and r == s):
+                    total += 8 * win + 16 * wout
+                total += 16 * wout + 8 * ends * wout
+    return total
+
+
+def scan_pass_bytes(st, nodes, edges):
+    """Bytes the scans cannot do without (light, heavy, and the vertex passes
+    before them: k_prep and k_flatten). Each scan streams one entry array and
+    nindex. The light one writes inMST and looks up the neighbours of all
+    entries that pass its weight test (both directions of what it keeps), the
+    heavy one a bit per vertex and, for what it keeps, the weight and two
+    parents. 16 per entry kept. The lightest heavy entries may be a list of the
+    light scan's (the heavy phase then has two lists)."""
+    w, rounds = st["wl_real"][1], st["rounds"][1]
+    mid = w[0] if len(list_starts(w, rounds)) > 1 else 0
+    light_kept, heavy_kept = st["scan_kept"][0] + mid, st["scan_kept"][1] - mid
+    rows = 4 * (nodes + 1)
+    light = rows + 5 * edges + 4 * min(edges, 2 * light_kept) + 16 * light_kept
+    heavy = rows + 4 * edges + nodes // 8 + (4 + 8 + 16) * heavy_kept if st["filtered"] else 0
+    return light, heavy, rows + 12 * nodes + (8 * nodes + nodes // 8 if st["filtered"] else 0)
+
+
+def solve_launches(nodes, edges, mode, quantile=1.0):
+    """Kernels of one solve (ecl_mst_run_device; `mode` heuristic, none, quantile
+    or learned, with weights loaded)."""
+    learned = mode == "learned" and edges >= 1 << 20
+    if mode == "learned" and not learned:
+        mode = "heuristic"
+    if edges <= 1 << 22 and not learned:
+        return 1  # k_cluster or k_group
+    dense = edges // nodes >= 4
+    share = {"none": 1.0, "quantile": min(1.0, quantile)}.get(
+        mode, (min(19, int(3.0 * nodes * 20 / edges)) + 1) / 21 if dense else 1.0)
+    lists = edges // nodes >= 6 and (nodes >= 1 << 23 or share * 0.5 * edges >= 3 << 20)
+    heavy = learned or (mode == "quantile" and quantile < 1) or (mode == "heuristic" and dense)
+    return (4  # k_prep, k_scan_light, k_round, k_round_tail
+            + 2 * learned  # k_sample, k_mlp_apply
+            + 3 * lists  # k_flatten, k_round, k_round_tail of the second light list
+            + 3 * (heavy and lists and nodes >= 1 << 23)  # and of the lightest heavy entries
+            + 4 * heavy)  # k_flatten, k_scan_heavy, k_round, k_round_tail
 
 
 def batch_leg(args, E, torch, dev, rank=0, world=1, dist=None, mode=None):
@@ -619,6 +692,7 @@ def main():
                               "slowdown": m / ablation[against]["ms"] if against in ablation else 1.0,
                               "inMST_identical": h == ref_hash}
             if name == "variant_base":
+                ablation[name]["round_bytes"] = round_kernel_bytes(st_a, g.nodes)
                 against = name
 
     # one extra solve counting the guarded atomics for the byte model
@@ -635,8 +709,8 @@ def main():
             # capture's DRAM traffic to a larger workload)
             print(json.dumps({"workload": args.workload, "ms_per_step": ms_step, "value": value,
                               "rounds": last["rounds"], "forest_weight": fw,
-                              "round_bytes": round_kernel_bytes(last, g.nodes, atomics=st_atom["atomics"]),
-                              "scan_bytes": scan_kernel_bytes(last, g.nodes, g.edges)}), flush=True)
+                              "round_bytes": round_pass_bytes(last, st_atom["atomics"]),
+                              "scan_bytes": sum(scan_pass_bytes(last, g.nodes, g.edges))}), flush=True)
         ctx.close()
         return
 
@@ -675,22 +749,22 @@ def main():
     d2h = g.edges
 
     peak, peak_kind = load_peaks()
-    rb = round_kernel_bytes(last, g.nodes, atomics=st_atom["atomics"])
-    # each scan streams one entry array and reads the other for the kept entries alone
-    unread = [4 * (g.edges - last["scan_kept"][p]) if p == 0 or last["filtered"] else 0 for p in range(2)]
-    sb = scan_kernel_bytes(last, g.nodes, g.edges) - sum(unread)
+    rb = round_pass_bytes(last, st_atom["atomics"])
+    scan_bytes = scan_pass_bytes(last, g.nodes, g.edges)
+    sb = sum(scan_bytes)
     r_ms = sum(round_ms) / len(round_ms)
     s_ms = sum(scan_ms) / len(scan_ms)
     kernels = {
         "rounds": {"bytes": rb, "ms": r_ms, "gbs": rb / (r_ms * 1e-3) / 1e9},
-        "scan": {"bytes": sb, "ms": s_ms, "gbs": sb / (s_ms * 1e-3) / 1e9},
+        "scan": {"bytes": sb, "ms": s_ms, "gbs": sb / (s_ms * 1e-3) / 1e9,
+                 "both_arrays_whole_bytes": scan_kernel_bytes(last, g.nodes, g.edges)},
     }
     # the worklist-build kernels alone (CUDA events around each scan launch)
     for p, (name, us) in enumerate((("light_scan", light_us), ("heavy_scan", heavy_us))):
         k_ms = sum(us) / len(us) / 1e3
         if p == 1 and not last["filtered"]:
             continue
-        kb = 4 * (g.nodes + 1) + 8 * g.edges + (g.edges if p == 0 else 0) + 16 * last["scan_kept"][p] - unread[p]
+        kb = scan_bytes[p]
         kernels[name] = {"bytes": kb, "ms": k_ms, "gbs": kb / (k_ms * 1e-3) / 1e9,
                          "frac": kb / (k_ms * 1e-3) / 1e9 / peak}
     dom = max(("rounds", "scan"), key=lambda k: kernels[k]["ms"])
@@ -706,7 +780,10 @@ def main():
     run = {"bytes": b_run, "ms": ms_step, "gbs": b_run / (ms_step * 1e-3) / 1e9,
            "frac": b_run / (ms_step * 1e-3) / 1e9 / peak,
            "what": "9m + 4n + 4 bytes (CSR read once, inMST written once) over the whole solve"}
-    roofline = {"bound": "hbm", "kernel": "k_round, k_round_tail" if dom == "rounds" else "k_scan_light, k_scan_heavy",
+    launches = solve_launches(g.nodes, g.edges, args.mode, args.quantile)
+    kernel = ("the rounds or the scans of the one launch" if launches == 1 else
+              "k_round, k_round_tail" if dom == "rounds" else "k_scan_light, k_scan_heavy")
+    roofline = {"bound": "hbm", "kernel": kernel,
                 "achieved": kernels[dom]["gbs"], "peak": peak, "unit": "GB/s",
                 "frac": kernels[dom]["gbs"] / peak, "peak_source": peak_kind, "traffic": traffic,
                 "per_kernel": kernels, "run": run}
@@ -804,9 +881,7 @@ def main():
                             "copy in overlaps the previous solve and copy back), wall clock over the steps",
                     "sync": {"value": world * g.edges / e2e_sync / 1e9, "ms": e2e_sync * 1e3,
                              "what": "one blocking ecl_mst_ctx_run_host call per step"}},
-            # per solve: k_prep, k_scan_light, k_round and k_round_tail, k_flatten and the two for the second
-            # light list, k_flatten, k_scan_heavy and the two; the learned schedule adds k_sample and k_mlp_apply
-            "gpu_launches": (13 if args.mode == "learned" else 11) * args.steps,
+            "gpu_launches": launches * args.steps,
             "ablation": ablation,
             "heuristic_schedule": ({"value": world * g.edges / (np.mean(heur_ms) * 1e-3) / 1e9,
                                     "ms": float(np.mean(heur_ms)),
