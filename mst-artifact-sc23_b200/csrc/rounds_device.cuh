@@ -717,7 +717,7 @@ __global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads
   if (b.W) {
     if (b.nseg) {
       bor_seg_load<kTailThreads>(s, st, b.nseg);
-      __syncthreads();
+      sy.sync();  // a CTA without entries publishes its new segment at once: not before all have read the old ones
     }
     bor_rounds<kTailThreads, kTailEpt, true, true>(a, b, sy, s, left);
     if (sy.rank == 0 && threadIdx.x == 0 && !left) st->rounds[a.phase] = b.r;
