@@ -91,7 +91,7 @@ struct ClMem {
   }
   // Adds `x` to the same shared-memory counter of every CTA (one thread).
   __device__ __forceinline__ void add_all(unsigned* counter, unsigned x) const {
-    if (kOne) *counter += x;
+    if (kOne || log == 0) *counter += x;
     else for (unsigned r = 0; r < (1u << log); r++) {
       unsigned a;
       asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(counter)), "r"(r));
