@@ -171,8 +171,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
 }
 
 // The rounds of one phase by the group, then the whole group again.
-template <class Sync>
-__device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, GroupSmem& sm) {
+__device__ bool group_rounds(const GroupArgs& g, int phase, int skip, GridSync& sy, GroupSmem& sm) {
   BorArgs a{};
   a.phase = phase;
   a.nodes = g.nodes;
@@ -209,8 +208,7 @@ __device__ bool group_rounds(const GroupArgs& g, int phase, int skip, Sync& sy, 
 
 // One solve; the control block's counters are zero. False if a barrier timed
 // out. Every thread of the group calls this.
-template <class Sync>
-__device__ bool group_solve(const GroupArgs& g, Sync& sy, GroupSmem& sm) {
+__device__ bool group_solve(const GroupArgs& g, GridSync& sy, GroupSmem& sm) {
   DevState* st = g.st;
   const unsigned rank = sy.rank, ctas = sy.active, tid = threadIdx.x;
   const unsigned gid = rank * kGroupThreads + tid, stride = ctas * kGroupThreads;

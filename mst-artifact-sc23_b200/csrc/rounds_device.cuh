@@ -202,11 +202,6 @@ struct ClusterSync {
     }
     return true;
   }
-  // The whole cluster again: the CTAs that left the rounds wait at its barrier.
-  __device__ __forceinline__ bool regroup(bool) {
-    active = ctas;
-    return sync();
-  }
 };
 
 __device__ __forceinline__ void bor_smem_init(BorSmem& s) {
