@@ -301,8 +301,7 @@ typedef struct ecl_mst_stats {
    * ms_scan), us_round from the device clock at the rounds' barriers:        */
   float us_scan[2][3];     /* [0]: {features + prep + light scan, features +
                               prep, light scan kernel}; [1]: {flatten + heavy
-                              scan, flatten (and the rounds of the heavy list
-                              set aside), heavy scan kernel}                   */
+                              scan, flatten, heavy scan kernel}                */
   float us_round[2][ECL_MAX_ROUNDS][2]; /* per round: offer pass, mark + roots  */
   int64_t wl_real[2][ECL_MAX_ROUNDS];   /* entries entering each round without
                                            the scans' null padding            */

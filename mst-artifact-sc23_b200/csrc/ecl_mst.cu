@@ -857,6 +857,8 @@ int fill_stats(ecl_mst_ctx* c, ecl_mst_stats* stats, bool timed, bool breakdown 
   for (int p = 0; p < 2; p++) {
     u64 prev = h.t_round_start[p];
     for (int r = 0; r < h.rounds[p] && r < ECL_MAX_ROUNDS; r++) {
+      for (int k : {2 * p, 2 * p + 1})  // a scan or a flattening pass lies before a list's rounds
+        if (h.t_list[k] && h.r_list[k] == r) prev = h.t_list[k];
       const u64 a = h.t_round[p][2 * r], b = h.t_round[p][2 * r + 1];
       if (a && prev) stats->us_round[p][r][0] = (a - prev) * 1e-3f;
       if (b && a) stats->us_round[p][r][1] = (b - a) * 1e-3f;
@@ -890,6 +892,16 @@ int fill_stats(ecl_mst_ctx* c, ecl_mst_stats* stats, bool timed, bool breakdown 
     float t05, t26;
     cudaEventElapsedTime(&t05, c->ev[0], c->ev[5]);
     cudaEventElapsedTime(&t26, c->ev[2], c->ev[6]);
+    // the rounds of the heavy list set aside run between flatten's events
+    const int mid_end = h.t_list[kListHeavy] ? h.r_list[kListHeavy] : h.rounds[1];
+    if (h.t_list[kListMid] && mid_end > 0 && mid_end <= ECL_MAX_ROUNDS) {
+      const u64 end = h.t_round[1][2 * mid_end - 2];
+      const float ms = end > h.t_list[kListMid] ? (float)(end - h.t_list[kListMid]) * 1e-6f : 0.f;
+      stats->ms_scan -= ms;
+      stats->ms_rounds += ms;
+      t23 -= ms;
+      t26 -= ms;
+    }
     stats->us_scan[0][0] = t01 * 1e3f;
     stats->us_scan[0][1] = t05 * 1e3f;
     stats->us_scan[0][2] = (t01 - t05) * 1e3f;

@@ -148,6 +148,8 @@ struct alignas(128) DevState {
   u64 t_round_start[2];
   u64 t_round[2][2 * ECL_MAX_ROUNDS];
   u64 t_step[kSteps];  // solves in one launch: ends of their steps (kStepStart ...)
+  u64 t_list[4];       // separate launches: start of a list's rounds (0 = none)
+  int r_list[4];       // and the phase's round it is
   ListCount lists[4];
   unsigned split_light;  // light entries up to this weight (as unsigned) go to list light 0
   unsigned split_heavy;  // heavy entries up to this weight go to list mid, if
@@ -182,6 +184,13 @@ struct alignas(128) DevState {
 // where the slots and parents of the vertices outgrow L2, so that every entry
 // the heavy scan keeps costs DRAM accesses (ER 16M 7.7 ms against 8.9, RMAT-25
 // 10.8 against 11.7; RMAT-22, in L2, 1.55 against 1.52).
+//   The line kMidNodes, times below and beyond it without and with what it
+// switches on: random graphs gain on both sides (degree 16, 7M vertices at the
+// 10 % quantile 2.94 and 2.22 ms, 9M 3.43 and 2.83, 12M 5.22 and 3.79, 16M 7.36 and
+// 5.34; degree 32 2.83 and 2.83, 3.61 and 3.78, 5.10 and 4.82, 8.28 and 6.87), power-law
+// graphs lose on both (RMAT-22 1.40 and 1.53, RMAT-23 2.52 and 3.00, RMAT-24 5.37 and
+// 5.77, heuristic; learned the same within 1.3 %). It lies where 20 bytes per
+// vertex pass L2's 126 MB.
 constexpr float kSplitLight = 0.5f, kSplitLightFar = 0.8f, kSplitHeavy = 2.0f;
 constexpr int kSplitMin = 3 << 20;
 constexpr int kMidNodes = 1 << 23;

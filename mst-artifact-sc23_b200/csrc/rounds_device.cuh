@@ -404,10 +404,10 @@ __device__ __forceinline__ void bor_roots_step(const BorArgs& a, const int (&v)[
 // Below some 10^5 entries a round is bound by its dependent L2 accesses (0.35
 // us a load or atomic) and barriers, so the loads that do not depend on each
 // other are issued together, the entries of a CTA with one tile stay in
-// registers from the offer to the mark pass (kKeep: not in k_round, whose 32
-// registers a thread they would spill, 2 % slower on RMAT-22), and where the
-// vertices are few for the threads at work the roots pass looks at all of them
-// instead of keeping a list.
+// registers from the offer to the mark pass (kKeep: not in k_round, which
+// spills 60 bytes of its 32 registers a thread as it is; 2 % slower on RMAT-22),
+// and where the vertices are few for the threads at work the roots pass looks at
+// all of them instead of keeping a list.
 template <int T, int E, bool kKeep, bool kLists, class Sync>
 __device__ __forceinline__ bool bor_rounds(const BorArgs& a, BorState& b, Sync& sy, BorSmem& s, bool& left) {
   constexpr int N = 2 * E;
@@ -682,6 +682,8 @@ __global__ void __launch_bounds__(kBorThreads, kBorBlocks) k_round(BorArgs a) {
   if (stamp) {
     if (b.r == 0) st->t_round_start[a.phase] = globaltimer_ns();
     if (b.W && b.r < ECL_MAX_ROUNDS) {
+      st->t_list[a.list] = globaltimer_ns();
+      st->r_list[a.list] = b.r;
       st->wl_count[a.phase][b.r] = b.W;
       st->wl_kept[a.phase][b.r] = st->lists[a.list].kept;
     }
