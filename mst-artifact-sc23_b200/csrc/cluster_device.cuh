@@ -164,7 +164,7 @@ __device__ void cl_scan(const ClArgs& g, const ClMem<kOne>& M, unsigned ctas, in
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       if (i < own) {
-        row_on([&](int r) { return __ldg(g.nindex + r); }, top, j0 + i, v, end);
+        row_on(g.nindex, top, j0 + i, v, end);
         bad |= (unsigned)nb[i] >= (unsigned)n;
         // one direction with a valid id (v < nb < n) as one unsigned compare
         if ((unsigned)nb[i] - (unsigned)v - 1u < (unsigned)(n - v - 1) && (KIND == kLight ? w[i] <= thr : w[i] > thr))
@@ -369,11 +369,15 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
     if (i != offsetof(DevState, graph) / sizeof(unsigned)) reinterpret_cast<unsigned*>(st)[i] = 0u;
   if (tid < 3) sm.total[tid] = 0;
   if (tid == 0) sm.cursor = 0;
-  sy.sync();
-  auto step_done = [&](int step) {
-    if (rank == 0 && tid == 0) st->t_step[step] = globaltimer_ns();
+  // a step's end is read before a barrier and stored after it: neither is waited for
+  const bool stamp = rank == 0 && tid == 0;
+  auto now = [&]() { return stamp ? globaltimer_ns() : 0ull; };
+  auto step_done = [&](int step, u64 t) {
+    if (stamp) st->t_step[step] = t;
   };
-  step_done(kStepStart);
+  u64 t = now();
+  sy.sync();
+  step_done(kStepStart, t);
   if (rank == 0 && g.batch && g.mode == ECL_THRESH_QUANTILE && g.quantile < 1.0f) {
     if (tid == 0) batch_quantile(st, g.eweight, m, g.quantile);
   } else if (rank == 0) {
@@ -397,7 +401,9 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
   }
   if (rank == 0 && tid == 0) bad |= __ldg(g.nindex) != 0 || __ldg(g.nindex + n) != m;
   if (bad) atomicOr(&st->error, kErrFormat);
+  t = now();
   sy.sync();
+  step_done(kStepPrep, t);
   if (ld_volatile(&st->error) & kErrFormat) return;  // only set before the barrier: the whole cluster
   const int thr = (int)ld_volatile((const unsigned*)&st->threshold);
   const int filtered = (int)ld_volatile((const unsigned*)&st->filtered);
@@ -406,11 +412,9 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
   int4* l0 = g.wl0 + region;
   int4* l1 = g.wl1 + region;
   unsigned pass_no = 0;
-  step_done(kStepPrep);
   cl_scan<kLight>(g, M, ctas, thr, l0, sm);
   __syncthreads();
   cl_rounds(g, M, sy, 0, -1, l0, l1, pass_no, sm);
-  step_done(kStepLight);
   if (!filtered) return;
   __syncthreads();
   if (tid == 0) sm.cursor = 0;
@@ -427,13 +431,13 @@ __device__ void cl_solve(const ClArgs& g, ClusterSync& sy, const ClMem<kOne>& M,
     const unsigned same = __popc(__match_any_sync(0xffffffffu, r));
     if (same == __reduce_max_sync(0xffffffffu, same)) st->giant = r;  // any of the largest groups
   }
+  t = now();
   sy.sync();
+  step_done(kStepFlatten, t);
   const int giant = (int)ld_volatile((const unsigned*)&st->giant);
-  step_done(kStepFlatten);
   cl_scan<kHeavy>(g, M, ctas, thr, l0, sm);
   __syncthreads();
   cl_rounds(g, M, sy, 1, giant, l0, l1, pass_no, sm);
-  step_done(kStepHeavy);
 }
 
 template <bool kOne>

@@ -871,13 +871,17 @@ int fill_stats(ecl_mst_ctx* c, ecl_mst_stats* stats, bool timed, bool breakdown 
     cudaEventElapsedTime(&stats->ms_total, c->ev[0], c->ev[4]);
     auto us = [](u64 from, u64 to) { return from && to > from ? (float)(to - from) * 1e-3f : 0.f; };
     const u64 *t = h.t_step, *r = h.t_round_start;
+    auto end = [&](int p) {  // of the phase's rounds
+      const int last = std::min(h.rounds[p], ECL_MAX_ROUNDS) - 1;
+      return last < 0 ? r[p] : h.t_round[p][2 * last];
+    };
     float(*sc)[3] = stats->us_scan;
     sc[0][1] = us(t[kStepStart], t[kStepPrep]);
     sc[0][2] = us(t[kStepPrep], r[0]);
-    sc[1][1] = us(t[kStepLight], t[kStepFlatten]);
+    sc[1][1] = t[kStepFlatten] ? us(end(0), t[kStepFlatten]) : 0.f;
     sc[1][2] = us(t[kStepFlatten], r[1]);
     for (int p = 0; p < 2; p++) sc[p][0] = sc[p][1] + sc[p][2];
-    stats->ms_rounds = (us(r[0], t[kStepLight]) + us(r[1], t[kStepHeavy])) * 1e-3f;
+    stats->ms_rounds = (us(r[0], end(0)) + us(r[1], end(1))) * 1e-3f;
     stats->ms_scan = std::max(0.f, stats->ms_total - stats->ms_rounds);
   } else if (timed) {
     float t01, t12, t23, t34, t04;

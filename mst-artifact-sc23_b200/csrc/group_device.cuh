@@ -63,6 +63,16 @@ __device__ __forceinline__ void warp_rows(const int* nindex, int n, int jl, int 
   }
 }
 
+// row_on over the CSR itself. The search is out of line: in line at every entry of
+// a scan it cost the one-cluster solve of 1000 vertices 1 us of 72, by its size.
+__device__ __noinline__ int last_row_of(const int* nindex, int lo, int hi, int j) {
+  return last_row([&](int r) { return __ldg(nindex + r); }, lo, hi, j);
+}
+__device__ __forceinline__ void row_on(const int* nindex, int top, int j, int& v, int& end) {
+  row_on([&](int r) { return __ldg(nindex + r); }, [&](int lo, int hi) { return last_row_of(nindex, lo, hi, j); }, top,
+         j, v, end);
+}
+
 // initWL by a group: every thread takes four consecutive entries, looks for
 // the row of the first between the rows its warp spans, and walks on from
 // there; appends as tuples, in chunks of slots the CTA's warps share.
@@ -116,7 +126,7 @@ __device__ void group_scan(const GroupArgs& g, unsigned rank, unsigned ctas, Gro
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       if (i < own) {
-        row_on([&](int r) { return __ldg(g.nindex + r); }, top, j0 + i, v, end);
+        row_on(g.nindex, top, j0 + i, v, end);
         bad |= (unsigned)nb[i] >= (unsigned)n;
         // one direction with a valid id (v < nb < n) as one unsigned compare
         if ((unsigned)nb[i] - (unsigned)v - 1u < (unsigned)(n - v - 1) && (KIND == kLight ? w[i] <= thr : w[i] > thr))
@@ -214,10 +224,14 @@ __device__ bool group_solve(const GroupArgs& g, GridSync& sy, GroupSmem& sm) {
   const unsigned gid = rank * kGroupThreads + tid, stride = ctas * kGroupThreads;
   const int n = g.nodes, m = g.edges;
   if (m == 0) return true;
-  auto step_done = [&](int step) {
-    if (rank == 0 && tid == 0) st->t_step[step] = globaltimer_ns();
+  // a step's end is read before a barrier and stored after it: neither is waited for
+  const bool stamp = rank == 0 && tid == 0;
+  auto now = [&]() { return stamp ? globaltimer_ns() : 0ull; };
+  auto step_done = [&](int step, u64 t) {
+    if (stamp) st->t_step[step] = t;
   };
-  step_done(kStepStart);
+  u64 t = now();
+  step_done(kStepStart, t);
   if (rank == 0) {
     PrepArgs pa{};
     pa.nodes = n;
@@ -239,14 +253,14 @@ __device__ bool group_solve(const GroupArgs& g, GridSync& sy, GroupSmem& sm) {
   }
   if (gid == 0) bad |= __ldg(g.nindex) != 0 || __ldg(g.nindex + n) != m;
   if (bad) atomicOr(&st->error, kErrFormat);
+  t = now();
   if (!sy.sync()) return false;
+  step_done(kStepPrep, t);
   if (ld_volatile(&st->error) & kErrFormat) return true;  // only set before the barrier: the whole group
-  step_done(kStepPrep);
   group_scan<kLight>(g, rank, ctas, sm);
   if (!sy.sync()) return false;
   const int filtered = st->filtered;
   if (!group_rounds(g, 0, -1, sy, sm)) return false;
-  step_done(kStepLight);
   if (!filtered) return true;
   // parent[v] = root(v), and the tree most entries point into (a vote of 32)
   for (unsigned v = gid; v < (unsigned)n; v += stride) {
@@ -262,14 +276,13 @@ __device__ bool group_solve(const GroupArgs& g, GridSync& sy, GroupSmem& sm) {
     const unsigned same = __popc(__match_any_sync(0xffffffffu, r));
     if (same == __reduce_max_sync(0xffffffffu, same)) st->giant = r;  // any of the largest groups
   }
+  t = now();
   if (!sy.sync()) return false;
+  step_done(kStepFlatten, t);
   const int giant = (int)ld_volatile((const unsigned*)&st->giant);
-  step_done(kStepFlatten);
   group_scan<kHeavy>(g, rank, ctas, sm);
   if (!sy.sync()) return false;
-  if (!group_rounds(g, 1, giant, sy, sm)) return false;
-  step_done(kStepHeavy);
-  return true;
+  return group_rounds(g, 1, giant, sy, sm);
 }
 
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) k_group(GroupArgs g) {

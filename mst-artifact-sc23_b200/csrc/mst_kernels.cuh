@@ -127,9 +127,9 @@ struct ListCount {
 };
 
 // Times (globaltimer) of a solve in one launch, which has no events between its
-// steps: its start, and the ends of prep, the light phase's rounds, flatten and
-// the heavy phase's rounds (the scans end where t_round_start is).
-enum : int { kStepStart = 0, kStepPrep, kStepLight, kStepFlatten, kStepHeavy, kSteps };
+// steps: its start, and the ends of prep and flatten (the scans end where
+// t_round_start is, the rounds with the last offer pass).
+enum : int { kStepStart = 0, kStepPrep, kStepFlatten, kSteps };
 
 // Control block of one solve, zeroed before every solve.
 struct alignas(128) DevState {
@@ -254,29 +254,31 @@ __device__ __forceinline__ int ld_ca(const int* p) {
   return v;
 }
 
-// On from row v, whose entries end at `end`, to the row of entry j, which is at
-// most `top`: first(r) is row r's first entry. A few rows are looked at one by
-// one. A longer run is one of empty rows, of any length, and is bisected: a
-// million isolated vertices between two entries of a thread, walked row by row,
-// took 50 ms a scan.
-constexpr int kRowSteps = 4;
+// The last of the rows lo .. hi that starts at or before entry j: first(r) is
+// row r's first entry, and row lo does.
 template <class First>
-__device__ __forceinline__ void row_on(First first, int top, int j, int& v, int& end) {
+__device__ __forceinline__ int last_row(First first, int lo, int hi, int j) {
+  while (lo < hi) {
+    const int mid = lo + ((hi - lo + 1) >> 1);
+    if (first(mid) <= j) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// On from row v, whose entries end at `end`, to the row of entry j, which is at
+// most `top`. A few rows are looked at one by one. A longer run is one of empty
+// rows, of any length, and is bisected (last(lo, hi)): a million isolated
+// vertices between two entries of a thread, walked row by row, took 50 ms a scan.
+constexpr int kRowSteps = 4;
+template <class First, class Last>
+__device__ __forceinline__ void row_on(First first, Last last, int top, int j, int& v, int& end) {
   for (int k = 0; j >= end && v < top; k++) {
-    if (k == kRowSteps) {
-      int lo = v + 1, hi = top;  // row v + 1 starts at `end`
-      while (lo < hi) {
-        const int mid = lo + ((hi - lo + 1) >> 1);
-        if (first(mid) <= j) lo = mid;
-        else hi = mid - 1;
-      }
-      v = lo - 1;
-    }
+    if (k == kRowSteps) v = last(v + 1, top) - 1;  // row v + 1 starts at `end`
     v++;
     end = v < top ? first(v + 1) : INT_MAX;
   }
 }
-
 // ---- mbarriers and bulk asynchronous copies (cp.async.bulk, no multicast)
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);

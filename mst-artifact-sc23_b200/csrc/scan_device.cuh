@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocks) k_scan_light(ScanAr
         unsigned cls = 0xffffu;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          row_on(first, top, j0 + at + i, row, end);
+          const int j = j0 + at + i;
+          row_on(first, [&](int lo, int hi) { return last_row(first, lo, hi, j); }, top, j, row, end);
           const int v = rows.lo + row;
           e[i] = make_int4(v, ends[i], data[at + i], j0 + at + i);
           const bool on = (mask >> (4 * g + i)) & 1u;
