@@ -244,7 +244,7 @@ constexpr size_t tree_bits_bytes(int64_t nodes) { return (size_t)(nodes + 31) / 
 int64_t first_v_entries(int64_t edges) { return edges / kGran + 2; }
 
 int enqueue_prep(const PrepArgs& pa, int sm_count, cudaStream_t s, const cudaAccessPolicyWindow* win = nullptr) {
-  const int grid = (int)std::min<int64_t>((pa.nodes + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
+  const int grid = (int)std::min<int64_t>(((int64_t)pa.nodes + kThreads - 1) / kThreads, (int64_t)sm_count * 16);
   return launch_ex(k_prep, std::max(grid, 1), kThreads, 0, s, false, win, pa);
 }
 

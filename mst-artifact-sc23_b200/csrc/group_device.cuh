@@ -51,7 +51,7 @@ __device__ __forceinline__ void warp_rows(const int* nindex, int n, int jl, int 
   int len_l = n, len_h = n;
   lo = hi = 0;
   while (len_l > 1 || len_h > 1) {
-    const int sl = (len_l + 31) >> 5, sh = (len_h + 31) >> 5;
+    const int sl = (int)(((unsigned)len_l + 31u) >> 5), sh = (int)(((unsigned)len_h + 31u) >> 5);  // n up to INT_MAX
     const int pl = lane * sl, ph = lane * sh;
     const bool bl = pl < len_l && (lane == 0 || __ldg(nindex + lo + pl) <= jl);
     const bool bh = ph < len_h && (lane == 0 || __ldg(nindex + hi + ph) <= jh);
